@@ -40,11 +40,11 @@ __global__ void __launch_bounds__(256) k_adj_stage(AdjStageParams<T> p) {
   if (i >= p.nx || j >= p.ny) return;
   constexpr int V = DIM + 2;
   constexpr int P = DIM + 1;
-  const long long nxy = (long long)p.nx * p.ny;
-  const long long l = i + (long long)p.nx * j + nxy * k;
+  const long long nxy = (long long)p.px * p.ny;
+  const long long l = i + (long long)p.px * j + nxy * k;
   const int pos[3] = {i, j, k};
   const int nn[3] = {p.nx, p.ny, p.nz};
-  const long long sd[3] = {1, p.nx, nxy};
+  const long long sd[3] = {1, p.px, nxy};
   const T scale = p.first ? p.hb_in : T(1);
   T acc[V];
 #pragma unroll
@@ -103,11 +103,11 @@ __global__ void __launch_bounds__(256) k_adj_filter(AdjFilterParams<T> p) {
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
   if (i >= p.nx || j >= p.ny) return;
-  const long long nxy = (long long)p.nx * p.ny;
-  const long long l = i + (long long)p.nx * j + nxy * k;
+  const long long nxy = (long long)p.px * p.ny;
+  const long long l = i + (long long)p.px * j + nxy * k;
   const int pos = p.dir == 0 ? i : (p.dir == 1 ? j : k);
   const int n = p.dir == 0 ? p.nx : (p.dir == 1 ? p.ny : p.nz);
-  const long long sd = p.dir == 0 ? 1 : (p.dir == 1 ? (long long)p.nx : nxy);
+  const long long sd = p.dir == 0 ? 1 : (p.dir == 1 ? (long long)p.px : nxy);
   const double* row = trans_row(p.op, pos, n);
   for (int v = 0; v < p.V; ++v) {
     T f = T(0);

@@ -77,7 +77,7 @@ __device__ __forceinline__ T dop_t(const OpTable& op, const T* __restrict__ g, l
 template <typename T, int DIM>
 __global__ void __launch_bounds__(256) k_adjg_flux(AdjGenParams<T> p) {
   const StageParams<T>& f = p.f;
-  const long long n = (long long)f.nx * f.ny * f.nz;
+  const long long n = (long long)f.px * f.ny * f.nz;  // the rows' pads included (zeros)
   constexpr int V = DIM + 2, P = DIM + 1;
   for (long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x; l < n; l += (long long)gridDim.x * blockDim.x) {
     T w[V];
@@ -119,11 +119,11 @@ __global__ void __launch_bounds__(256) k_adjg_stage(AdjGenParams<T> p) {
   const int k = blockIdx.z;
   if (i >= f.nx || j >= f.ny) return;
   constexpr int V = DIM + 2, P = DIM + 1;
-  const long long nxy = (long long)f.nx * f.ny;
-  const long long l = i + (long long)f.nx * j + nxy * k;
+  const long long nxy = (long long)f.px * f.ny;
+  const long long l = i + (long long)f.px * j + nxy * k;
   const int pos[3] = {i, j, k};
   const int nn[3] = {f.nx, f.ny, f.nz};
-  const long long sd[3] = {1, f.nx, nxy};
+  const long long sd[3] = {1, f.px, nxy};
   T acc[V];
 #pragma unroll
   for (int v = 0; v < V; ++v) {
@@ -201,11 +201,11 @@ __global__ void __launch_bounds__(256) k_adjg_filter(AdjGenFilterParams<T> p) {
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
   if (i >= p.nx || j >= p.ny) return;
-  const long long nxy = (long long)p.nx * p.ny;
-  const long long l = i + (long long)p.nx * j + nxy * k;
+  const long long nxy = (long long)p.px * p.ny;
+  const long long l = i + (long long)p.px * j + nxy * k;
   const int pos = p.dir == 0 ? i : (p.dir == 1 ? j : k);
   const int n = p.dir == 0 ? p.nx : (p.dir == 1 ? p.ny : p.nz);
-  const long long sd = p.dir == 0 ? 1 : (p.dir == 1 ? (long long)p.nx : nxy);
+  const long long sd = p.dir == 0 ? 1 : (p.dir == 1 ? (long long)p.px : nxy);
   const int R = max(p.op.h, max(p.op.S - 1, p.op.nb - 1));
   for (int v = 0; v < p.V; ++v) {
     T acc = T(0);
@@ -270,8 +270,8 @@ __global__ void k_adjg_bc(BcParams<T> p) {
     const int i = p.lo[0] + (int)(lb % p.nb[0]);
     const int j = p.lo[1] + (int)((lb / p.nb[0]) % p.nb[1]);
     const int k = p.lo[2] + (int)(lb / ((long long)p.nb[0] * p.nb[1]));
-    const long long l = i + (long long)p.nx * (j + (long long)p.ny * k);
-    if (p.iblank && p.iblank[l] == 1) continue;
+    const long long row = j + (long long)p.ny * k, l = i + p.px * row, lu = i + p.nx * row;
+    if (p.iblank && p.iblank[lu] == 1) continue;
     const int P = p.nd + 1;
     double tmp[kMaxVars];
     bool scat[kMaxVars];
@@ -292,16 +292,16 @@ __global__ void k_adjg_bc(BcParams<T> p) {
       // slip wall: u_out = J Minv Z Met u (Z zeroes the wall-normal contravariant component);
       // its transpose Met^T Z Minv^T J acts on the velocity adjoint at the point
       scat[0] = scat[P] = true;
-      const double jac = p.jac[l];
+      const double jac = p.jac[lu];
       double vc[3] = {0.0, 0.0, 0.0};
       for (int a = 0; a < p.nd; ++a) {
         double s = 0.0;
-        for (int q = 0; q < p.nd; ++q) s += p.minv[q * 3 + a][l] * jac * tmp[1 + q];
+        for (int q = 0; q < p.nd; ++q) s += p.minv[q * 3 + a][lu] * jac * tmp[1 + q];
         vc[a] = a == p.dir ? 0.0 : s;
       }
       for (int q = 0; q < p.nd; ++q) {
         double s = 0.0;
-        for (int a = 0; a < p.nd; ++a) s += p.met[a * 3 + q][l] * vc[a];
+        for (int a = 0; a < p.nd; ++a) s += p.met[a * 3 + q][lu] * vc[a];
         p.y[1 + q][l] = (T)s;
       }
     }
@@ -355,7 +355,7 @@ int grid1(long long n) {
 
 template <typename T>
 cudaError_t launch_adjg_stage(const AdjGenParams<T>& p, cudaStream_t s) {
-  const long long n = (long long)p.f.nx * p.f.ny * p.f.nz;
+  const long long n = (long long)p.f.px * p.f.ny * p.f.nz;
   dim3 blk(32, 8, 1);
   dim3 grd((p.f.nx + 31) / 32, (p.f.ny + 7) / 8, p.f.nz);
   if (p.f.dim == 2) {

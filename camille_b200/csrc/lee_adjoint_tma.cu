@@ -124,8 +124,8 @@ __global__ void __launch_bounds__(256) k_adj_tma(const __grid_constant__ AdjMaps
     for (int x = 0; x < 3; ++x) jm[x] = JMF ? slot[(5 + d * 3 + x) * FBP + o] : p.jm[d * 3 + x].c;
   };
 
-  const unsigned nxy = (unsigned)p.nx * (unsigned)p.ny;
-  const unsigned lij = (unsigned)i + (unsigned)p.nx * (unsigned)j;
+  const unsigned nxy = (unsigned)p.px * (unsigned)p.ny;
+  const unsigned lij = (unsigned)i + (unsigned)p.px * (unsigned)j;
   // per-point results of the last planes: L^T restricted to xi and eta, and w at the point; and
   // G^zeta at the point over the planes the zeta stencil reads (zq[0] the oldest)
   T rq[kAH + 1][5], wq[kAH + 1][5], zq[2 * kAH + 1][5];

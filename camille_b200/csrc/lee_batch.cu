@@ -120,14 +120,14 @@ __device__ __forceinline__ void cp_wait() {
 // NT threads: cp.async inside the block, zeros outside it; one commit group per row (empty
 // when the row is outside the block, so the group count stays one per row).
 template <typename T, int V, int TX, int H, int NT = TX>
-__device__ __forceinline__ void issue_row(T* ring, int slot, const T* const* fields, int r, int x0, int nx, int ny,
-                                          int tid) {
+__device__ __forceinline__ void issue_row(T* ring, int slot, const T* const* fields, int r, int x0, int nx, int px,
+                                          int ny, int tid) {
   constexpr int W = TX + 2 * H;
   if (r >= 0 && r < ny) {
 #pragma unroll
     for (int v = 0; v < V; ++v) {
       T* dst = ring + ((long long)slot * V + v) * W;
-      const T* src = fields[v] + (long long)r * nx;
+      const T* src = fields[v] + (long long)r * px;
       for (int cc = tid; cc < W; cc += NT) {
         const int gx = x0 - H + cc;
         if (gx >= 0 && gx < nx) cp_async(dst + cc, src + gx);
@@ -168,21 +168,21 @@ __device__ __forceinline__ void batch_stage_run(const StageParams<T>* __restrict
       __syncthreads();
       if (tid == 0) cur = it.x;
     }
-    const int nx = P.nx, ny = P.ny, x0 = it.y, ys = it.z, ye = it.w;
+    const int nx = P.nx, px = P.px, ny = P.ny, x0 = it.y, ys = it.z, ye = it.w;
     const T* const* zin = P.zin;
     // prologue: rows ys - H .. ys + H + PF - 1
     for (int r = ys - H; r < ys + H + PF; ++r)
-      issue_row<T, V, SW, H, TX>(ring, (r + NS) % NS, zin, r, x0, nx, ny, tid);
+      issue_row<T, V, SW, H, TX>(ring, (r + NS) % NS, zin, r, x0, nx, px, ny, tid);
     PointIn<T, 2> in_cur[CX], in_nxt[CX];
 #pragma unroll
     for (int m = 0; m < CX; ++m)
-      if (x0 + tid + m * TX < nx) gather<T, 2, COMP, TR>(P, (long long)ys * nx + x0 + tid + m * TX, in_cur[m]);
+      if (x0 + tid + m * TX < nx) gather<T, 2, COMP, TR>(P, (long long)ys * px + x0 + tid + m * TX, in_cur[m]);
     for (int j = ys; j < ye; ++j) {
-      issue_row<T, V, SW, H, TX>(ring, (j + H + PF + NS) % NS, zin, j + H + PF, x0, nx, ny, tid);
+      issue_row<T, V, SW, H, TX>(ring, (j + H + PF + NS) % NS, zin, j + H + PF, x0, nx, px, ny, tid);
 #pragma unroll
       for (int m = 0; m < CX; ++m)
         if (x0 + tid + m * TX < nx && j + 1 < ye)
-          gather<T, 2, COMP, TR>(P, (long long)(j + 1) * nx + x0 + tid + m * TX, in_nxt[m]);
+          gather<T, 2, COMP, TR>(P, (long long)(j + 1) * px + x0 + tid + m * TX, in_nxt[m]);
       cp_wait<PF>();
       __syncthreads();
       int so[2 * H + 1];
@@ -200,7 +200,7 @@ __device__ __forceinline__ void batch_stage_run(const StageParams<T>* __restrict
             D[v][1] = dop_ring<T, kFdH, 3, NS>(w, ring, so, V * W, v * W + cl + H, j, ny);
             q[v] = *c0;
           }
-          rhs_update<T, 2, COMP, TR>(P, (long long)j * nx + i, i, j, 0, D, q, in_cur[m]);
+          rhs_update<T, 2, COMP, TR>(P, (long long)j * px + i, i, j, 0, D, q, in_cur[m]);
         }
         in_cur[m] = in_nxt[m];
       }
@@ -241,7 +241,7 @@ __device__ __forceinline__ void batch_filter_run(const BatchFilterInst<T>* __res
       __syncthreads();
       if (tid == 0) cur = it.x;
     }
-    const int nx = P.nx, ny = P.ny, x0 = it.y, ys = it.z, ye = it.w;
+    const int nx = P.nx, px = P.px, ny = P.ny, x0 = it.y, ys = it.z, ye = it.w;
     const T* const* xf = P.x + vb;
     const int i = x0 + tid;
     const bool col = i < nx;
@@ -255,13 +255,13 @@ __device__ __forceinline__ void batch_filter_run(const BatchFilterInst<T>* __res
       for (int q = 0; q <= H; ++q) dq[v][q] = T(0);
     }
     T err_nxt[V];
-    for (int r = ys - H; r < ys - H + PF; ++r) issue_row<T, V, TX, H>(X, (r + NX) % NX, xf, r, x0, nx, ny, tid);
+    for (int r = ys - H; r < ys - H + PF; ++r) issue_row<T, V, TX, H>(X, (r + NX) % NX, xf, r, x0, nx, px, ny, tid);
     for (int r = ys - H; r < ye + H; ++r) {
-      issue_row<T, V, TX, H>(X, (r + PF + NX) % NX, xf, r + PF, x0, nx, ny, tid);
+      issue_row<T, V, TX, H>(X, (r + PF + NX) % NX, xf, r + PF, x0, nx, px, ny, tid);
       const int j = r - H;  // the row finished in this iteration
       if (COMP && col && j >= ys && j < ye) {
 #pragma unroll
-        for (int v = 0; v < V; ++v) err_nxt[v] = P.err[vb + v][(long long)j * nx + i];
+        for (int v = 0; v < V; ++v) err_nxt[v] = P.err[vb + v][(long long)j * px + i];
       }
       cp_wait<PF>();
       __syncthreads();  // state row r landed for every thread
@@ -284,7 +284,7 @@ __device__ __forceinline__ void batch_filter_run(const BatchFilterInst<T>* __res
         }
       }
       if (col && j >= ys && j < ye) {
-        const long long l = (long long)j * nx + i;
+        const long long l = (long long)j * px + i;
         const T* xrow = X + (long long)((j + NX) % NX) * V * W + tid + H;
 #pragma unroll
         for (int v = 0; v < V; ++v) {

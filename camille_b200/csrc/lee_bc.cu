@@ -55,8 +55,9 @@ __global__ void k_bc(BcParams<T> p) {
     const int i = p.lo[0] + (int)(lb % p.nb[0]);
     const int j = p.lo[1] + (int)((lb / p.nb[0]) % p.nb[1]);
     const int k = p.lo[2] + (int)(lb / ((long long)p.nb[0] * p.nb[1]));
-    const long long l = i + (long long)p.nx * (j + (long long)p.ny * k);
-    if (p.iblank && p.iblank[l] == 1) continue;
+    // l: the point in the state fields (rows px apart); lu: in the setup fields
+    const long long row = j + (long long)p.ny * k, l = i + p.px * row, lu = i + p.nx * row;
+    if (p.iblank && p.iblank[lu] == 1) continue;
     const int P = p.nd + 1;
     double out[kMaxVars];
     if (p.kind == LEE_BC_NEUMANN) {
@@ -70,7 +71,7 @@ __global__ void k_bc(BcParams<T> p) {
       for (int v = 0; v < p.V; ++v) out[v] = 0.0;
     } else if (p.kind == LEE_BC_DIRICHLET_HARMONICWAVE) {
       for (int v = 0; v < p.V; ++v) out[v] = 0.0;
-      const double x[3] = {p.xyz[0][l], p.xyz[1][l], p.xyz[2][l]};
+      const double x[3] = {p.xyz[0][lu], p.xyz[1][lu], p.xyz[2][lu]};
       const double t = p.t_tab ? p.t_tab[(long long)*p.ctr * p.t_stride] : p.t;
       double ws, wu, wp;
       wave_eval(p.wave, x, t, &ws, &wu, &wp);
@@ -84,14 +85,14 @@ __global__ void k_bc(BcParams<T> p) {
       for (int q = 0; q < p.nd; ++q) vel[q] = ld<T, PAIR>(p, 1 + q, l);
       for (int a = 0; a < p.nd; ++a) {
         double s = 0.0;
-        for (int q = 0; q < p.nd; ++q) s = __dadd_rn(s, __dmul_rn(p.met[a * 3 + q][l], vel[q]));
+        for (int q = 0; q < p.nd; ++q) s = __dadd_rn(s, __dmul_rn(p.met[a * 3 + q][lu], vel[q]));
         vc[a] = s;
       }
       vc[p.dir] = 0.0;
-      const double jac = p.jac[l];
+      const double jac = p.jac[lu];
       for (int q = 0; q < p.nd; ++q) {
         double s = 0.0;
-        for (int a = 0; a < p.nd; ++a) s = __dadd_rn(s, __dmul_rn(p.minv[q * 3 + a][l], vc[a]));
+        for (int a = 0; a < p.nd; ++a) s = __dadd_rn(s, __dmul_rn(p.minv[q * 3 + a][lu], vc[a]));
         out[1 + q] = __dmul_rn(s, jac);
       }
     }
@@ -166,7 +167,7 @@ __global__ void k_ovs_gather(OvsParams<T> p) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= p.n) return;
   const int d = p.db[r];
-  const long long nx = p.nx[d], nxy = nx * p.ny[d];
+  const long long nx = p.px[d], nxy = nx * p.ny[d];
   const long long base = p.dl[r];
   const double* cf = p.wt + (long long)r * p.W;
   double acc[kMaxVars] = {0.0, 0.0, 0.0, 0.0, 0.0};

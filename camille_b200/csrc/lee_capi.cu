@@ -10,11 +10,12 @@ using namespace lee;
 namespace {
 
 // FP64 -> (y, e) with y = fl32(x) and e = fl32(x - y): the compensated pair of an uploaded state
-__global__ void k_split(long long n, float* y, float* e, const double* in) {
+__global__ void k_split(long long n, int nx, int px, float* y, float* e, const double* in) {
   for (long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x; l < n; l += (long long)gridDim.x * blockDim.x) {
     const float r = (float)in[l];
-    y[l] = r;
-    e[l] = (float)(in[l] - (double)r);
+    const long long q = row_pos(l, nx, px);
+    y[q] = r;
+    e[q] = (float)(in[l] - (double)r);
   }
 }
 
@@ -361,16 +362,23 @@ int lee_upload_state(lee_ctx* c, int b, const double* const sol[5], int step, do
     for (long long l = 0; l < bk.N; ++l)
       if (sol[3][l] != 0.0) return fail(c, LEE_ERR_ARG, "2-D state must have w' = 0");
   double* tmp = nullptr;
-  if (c->comp) {
+  if (c->comp || bk.px != bk.nx) {
     const int rc = staging(c, &tmp);
     if (rc) return rc;
   }
   for (int v = 0; v < c->V; ++v) {
-    if (!c->comp) {
+    if (bk.px != bk.nx) {  // the rows' pads: zeros, whatever a diverged run left in them
+      CK(cudaMemsetAsync(bk.y[v], 0, (size_t)bk.NP * c->esz, c->stream));
+      if (c->comp) CK(cudaMemsetAsync(bk.comp[v], 0, (size_t)bk.NP * c->esz, c->stream));
+    }
+    if (!c->comp && bk.px == bk.nx) {
       CK(cudaMemcpyAsync(bk.y[v], sol[slot_of(c->V, v)], (size_t)bk.N * 8, cudaMemcpyHostToDevice, c->stream));
     } else {
       CK(cudaMemcpyAsync(tmp, sol[slot_of(c->V, v)], (size_t)bk.N * 8, cudaMemcpyHostToDevice, c->stream));
-      k_split<<<grid1d(bk.N), 256, 0, c->stream>>>(bk.N, (float*)bk.y[v], (float*)bk.comp[v], tmp);
+      if (c->comp)
+        k_split<<<grid1d(bk.N), 256, 0, c->stream>>>(bk.N, bk.nx, bk.px, (float*)bk.y[v], (float*)bk.comp[v], tmp);
+      else
+        launch_convert<double>(c->stream, bk.N, (double*)bk.y[v], tmp, bk.nx, bk.px);
       CK(cudaGetLastError());
     }
   }
@@ -391,16 +399,18 @@ int lee_download_state(lee_ctx* c, int b, double* const sol[5], int* step, doubl
   BlockData& bk = c->blk[(size_t)b];
   CK(cudaSetDevice(c->cfg.device));
   double* tmp = nullptr;
-  if (c->comp) {
+  if (c->comp || bk.px != bk.nx) {
     const int rc = staging(c, &tmp);
     if (rc) return rc;
   }
   for (int v = 0; v < c->V; ++v) {
-    if (!c->comp) {
+    if (!c->comp && bk.px == bk.nx) {
       CK(cudaMemcpyAsync(sol[slot_of(c->V, v)], bk.y[v], (size_t)bk.N * 8, cudaMemcpyDeviceToHost, c->stream));
     } else {
-      launch_to_double<float>(c->stream, bk.N, tmp, (const float*)bk.y[v],
-                                                             (const float*)bk.comp[v]);
+      if (c->comp)
+        launch_to_double<float>(c->stream, bk.N, tmp, (const float*)bk.y[v], (const float*)bk.comp[v], bk.nx, bk.px);
+      else
+        launch_to_double<double>(c->stream, bk.N, tmp, (const double*)bk.y[v], nullptr, bk.nx, bk.px);
       CK(cudaGetLastError());
       CK(cudaMemcpyAsync(sol[slot_of(c->V, v)], tmp, (size_t)bk.N * 8, cudaMemcpyDeviceToHost, c->stream));
     }
@@ -447,8 +457,8 @@ int lee_state_minmax(lee_ctx* c, double* mn, double* mx) {
   CK(cudaMemcpyAsync(c->d_report, init, sizeof init, cudaMemcpyHostToDevice, c->stream));
   for (auto& bk : c->blk)
     for (int v = 0; v < c->V; ++v)
-      CK(setup_state_minmax(bk.N, bk.y[v], c->comp ? bk.comp[v] : nullptr, c->comp, c->d_report + 2 * slot_of(c->V, v),
-                            c->stream));
+      CK(setup_state_minmax((long long)bk.ny * bk.nz, bk.nx, bk.px, bk.y[v], c->comp ? bk.comp[v] : nullptr, c->comp,
+                            c->d_report + 2 * slot_of(c->V, v), c->stream));
   double out[10];
   CK(cudaMemcpyAsync(out, c->d_report, sizeof out, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));

@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(256, PX * sizeof(T) == 16 ? 2 : 3)
 #pragma unroll
   for (int o = 0; o <= HF; ++o) wi[o] = V::w(P.w[0][HF + o]);
   const int cy = cls_of(min(j, P.ny - 1), P.ny, HF);
-  const bool vec_io = (P.nx % PX) == 0;  // global groups are 16-byte aligned
+  const bool vec_io = (P.px % PX) == 0;  // global groups are 16-byte aligned
   // xi closure points: the owner of a group skips them (cmask, bit q for point i + q), and after
   // the group stores each warp's lanes compute the closure points of the warp's rows, lane L
   // taking row task L / (2 HF) and closure point L % (2 HF) (left end first)
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(256, PX * sizeof(T) == 16 ? 2 : 3)
     // before this plane's work so that the load's latency overlaps it
     const int kf = DIM == 3 ? p - HF : 0;
     const bool fin = kf >= k0 && kf < k1 && j < P.ny && i < P.nx;
-    const unsigned long long l = (unsigned long long)i + (unsigned long long)P.nx * (j + (unsigned long long)P.ny * kf);
+    const unsigned long long l = (unsigned long long)i + (unsigned long long)P.px * (j + (unsigned long long)P.ny * kf);
     const bool whole = vec_io && i + PX <= P.nx;
     V ef = V::zero();
     if (COMP && fin) {

@@ -91,7 +91,9 @@ __global__ void __launch_bounds__(256, HF <= 4 ? 4 : 3) k_filter_pair(const __gr
   const int k1 = min(P.nz, k0 + P.k_chunk);
   const int tid = threadIdx.x, tx = tid % kPairLX, ty = tid / kPairLX;
   const int i = i0 + 2 * tx, j = j0 + ty;
-  const bool active = i < P.nx && j < P.ny;  // nx is even: both points of the pair or neither
+  // with an odd nx the last pair's second point is the row's pad (the pitch px is even): its xi
+  // weights are zero and the copies fill beyond nx with zeros, so its pad values stay zero
+  const bool active = i < P.nx && j < P.ny;
   const int plo = max(0, k0 - HF), phi = min(P.nz - 1, k1 - 1 + HF);
 
   if (tid == 0) {
@@ -115,7 +117,7 @@ __global__ void __launch_bounds__(256, HF <= 4 ? 4 : 3) k_filter_pair(const __gr
   {
     const int cxa = cls_of(min(i, P.nx - 1), P.nx, P.nb), cxb = cls_of(min(i + 1, P.nx - 1), P.nx, P.nb);
 #pragma unroll
-    for (int o = 0; o < NQ; ++o) wx[o] = make_float2(P.w[cxa][o], P.w[cxb][o]);
+    for (int o = 0; o < NQ; ++o) wx[o] = make_float2(P.w[cxa][o], i + 1 < P.nx ? P.w[cxb][o] : 0.f);
   }
   const int cy = cls_of(min(j, P.ny - 1), P.ny, P.nb);
   const int c = G::HX + 2 * tx;  // column of the pair's first point in a box row
@@ -141,8 +143,8 @@ __global__ void __launch_bounds__(256, HF <= 4 ? 4 : 3) k_filter_pair(const __gr
   };
 
   // point offsets fit 32 bits (the host checks the block size)
-  const unsigned nxy = (unsigned)P.nx * (unsigned)P.ny;
-  const unsigned lij = (unsigned)i + (unsigned)P.nx * (unsigned)j;
+  const unsigned nxy = (unsigned)P.px * (unsigned)P.ny;
+  const unsigned lij = (unsigned)i + (unsigned)P.px * (unsigned)j;
   // (the carried error may be read from and written to the same buffer: each point's error is
   // read by its owner before the owner writes the new one)
   const float* errp = P.err[v];
@@ -277,7 +279,7 @@ void filter_pair_box(int hf, int* bx, int* by, int* tx, int* ty) {
 
 cudaError_t launch_filter_pair(const FieldMaps& in, const TmaFilterParams<float>& p, int hf, int comp, int tiles,
                                int chunks, cudaStream_t s) {
-  if (p.nx % 2 != 0 || p.code[0] || (comp && (!p.err[0] || !p.comp[0]))) return cudaErrorInvalidValue;
+  if (p.px % 2 != 0 || p.code[0] || (comp && (!p.err[0] || !p.comp[0]))) return cudaErrorInvalidValue;
 #define LEE_PAIR_CASE(HF)                                                                            \
   if (hf == HF)                                                                                      \
     return comp ? go_filter_pair<HF, true>(in, p, tiles, chunks, s) : go_filter_pair<HF, false>(in, p, tiles, chunks, s);

@@ -36,7 +36,13 @@ struct Boundary {
 
 struct BlockData {
   int nx = 0, ny = 0, nz = 0;
-  long long N = 0;
+  long long N = 0;          // points
+  // The time loop's arrays (state, coefficients, closure codes, masks) keep their rows px points
+  // apart, NP = px ny nz points in all: px = nx, or nx rounded up to a 16-byte multiple where the
+  // TMA-staged kernels then apply (set_pitch). Pads hold zeros. The setup products below and every
+  // array of the C ABI have rows of nx.
+  int px = 0;
+  long long NP = 0;
   bool set = false, has_mean = false;
   std::vector<double> hx, hy, hz;
   std::vector<int> hib;
@@ -55,6 +61,11 @@ struct BlockData {
   int* d_iblank = nullptr;
   int8_t* d_code_fd[3] = {};
   int8_t* d_code_flt[3] = {};
+  // the same at the time loop's row pitch (aliases when px = nx), and p_bar (pads 1)
+  int* d_tiblank = nullptr;
+  int8_t* d_tcode_fd[3] = {};
+  int8_t* d_tcode_flt[3] = {};
+  double* d_tpbar = nullptr;
   bool has_holes = false;   // some point is BLANKED: hole closures and hole bypass
   bool has_iblank = false;  // some point is not NOTBLANKED (holes or receivers): CFL skips them
   // per-block clock (blocks advanced with their own time steps keep their own time)
@@ -92,6 +103,7 @@ struct BlockData {
   int tiles_x = 0, tiles_y = 0;
   int stage_chunk = 0, filter_chunk = 0;
   int filter_ry = 1;                  // rows per thread row of the scalar fused filter (1 or 2)
+  int filter_form = 0;                // lee_set_filter_form where the block can run it, else 0 (timed)
   bool filter_pair_ok = false;        // the two-point compensated filter (lee_filter_pair.cu) applies
   bool filter_pair = false;           // ... and runs the block's fused filter (form 3)
   int ptiles_x = 0, ptiles_y = 0;     // its tiles
@@ -311,7 +323,7 @@ int classify(lee_ctx* c, const double* d_field, long long N, double scale, doubl
 template <typename T>
 int make_coef(lee_ctx* c, BlockData& b, const double* d_field, double scale, Coef<T>* out);
 int upload(lee_ctx* c, double** d, const std::vector<double>& h);
-int alloc_fields(lee_ctx* c, void** f, long long N);
+int alloc_fields(lee_ctx* c, void** f, long long N);  // V zeroed fields of N points
 int slot_of(int V, int v);
 template <typename T>
 void fill_stage_common(lee_ctx* c, BlockData& b, StageParams<T>& p);
@@ -328,6 +340,7 @@ bool class_weights(const OpTable& op, int H, double* w, int stride);
 Tableau tableau(int rk);
 int compute_metrics(lee_ctx* c, BlockData& b);
 int build_sigma_field(lee_ctx* c, BlockData& b);
+void set_pitch(const lee_ctx* c, BlockData& b);
 template <typename T>
 int run_filter(lee_ctx* c, BlockData& b, void** in, void** err, void** comp_out, void** f0, void** f1,
                void*** result);
@@ -428,10 +441,11 @@ void** as_void(T** p) {
   return reinterpret_cast<void**>(p);
 }
 
+// FP64 rows of nx points -> out, its rows px apart; and back (n points in all)
 template <typename T>
-void launch_convert(cudaStream_t s, long long n, T* out, const double* in);
+void launch_convert(cudaStream_t s, long long n, T* out, const double* in, int nx = 1, int px = 1);
 template <typename T>
-void launch_to_double(cudaStream_t s, long long n, double* out, const T* y, const T* comp);
+void launch_to_double(cudaStream_t s, long long n, double* out, const T* y, const T* comp, int nx = 1, int px = 1);
 // flag = 1 when some value of the V fields f (and e, when given) of n elements of esz bytes is
 // not finite
 cudaError_t launch_nonfinite(cudaStream_t s, long long n, int V, size_t esz, void* const* f, void* const* e,

@@ -91,18 +91,18 @@ int adjoint_setup(lee_ctx* c) {
   {
     int nf = 0;
     for (int q = 0; q < 9; ++q) nf += (c->comp ? (const void*)b.cf_jm[q].p : (const void*)b.cd_jm[q].p) != nullptr;
-    a.tma = c->cfg.num_dim == 3 && a.dT.H == 2 && ((size_t)b.nx * c->esz) % 16 == 0 &&
-            (unsigned long long)b.N < (1ull << 32) && (nf == 0 || nf == 9);
+    a.tma = c->cfg.num_dim == 3 && a.dT.H == 2 && ((size_t)b.px * c->esz) % 16 == 0 &&
+            (unsigned long long)b.NP < (1ull << 32) && (nf == 0 || nf == 9);
     a.tma_jm = nf == 9;
     // the transposed filter through the fused filter kernel: its instantiated widths, rows of
     // 16-byte multiples (the TMA box), class rows within the parameter table
     const int H = a.fT.H;
     a.fused_filter = c->cfg.filter_scheme != LEE_FILTER_NONE && (H == 2 || H == 4 || H == 5) &&
-                     a.fT.E <= kTE && ((size_t)b.nx * c->esz) % 16 == 0 && (unsigned long long)b.N < (1ull << 32);
+                     a.fT.E <= kTE && ((size_t)b.px * c->esz) % 16 == 0 && (unsigned long long)b.NP < (1ull << 32);
   }
   int rc;
-  if ((rc = alloc_fields(c, a.lam, b.N)) || (rc = alloc_fields(c, a.mu, b.N)) || (rc = alloc_fields(c, a.kb[0], b.N)) ||
-      (rc = alloc_fields(c, a.kb[1], b.N)) || (rc = alloc_fields(c, a.ybar, b.N)))
+  if ((rc = alloc_fields(c, a.lam, b.NP)) || (rc = alloc_fields(c, a.mu, b.NP)) || (rc = alloc_fields(c, a.kb[0], b.NP)) ||
+      (rc = alloc_fields(c, a.kb[1], b.NP)) || (rc = alloc_fields(c, a.ybar, b.NP)))
     return rc;
   bool spg = false;
   for (auto& z : b.bnd) spg |= z.kind == LEE_SPONGE_FREUND_AMBIENT;
@@ -128,6 +128,7 @@ int adjoint_step(lee_ctx* c, double dt, const double* amps, double* gbar) {
     TmaFilterParams<T> fp;
     memset(&fp, 0, sizeof fp);
     fp.nx = b.nx; fp.ny = b.ny; fp.nz = b.nz;
+    fp.px = b.px;
     fp.V = V;
     fp.tiles_x = b.tiles_x;
     // the scalar fused filter's form and chunk (the forward filter may run the two-point kernel)
@@ -180,7 +181,9 @@ int adjoint_step(lee_ctx* c, double dt, const double* amps, double* gbar) {
     for (int q = 0; q < nd; ++q) {
       AdjFilterParams<T> fp;
       memset(&fp, 0, sizeof fp);
-      fp.nx = b.nx; fp.ny = b.ny; fp.nz = b.nz; fp.V = V; fp.dir = dirs[q]; fp.last = q == nd - 1;
+      fp.nx = b.nx; fp.ny = b.ny; fp.nz = b.nz; fp.V = V;
+      fp.px = b.px;
+      fp.dir = dirs[q]; fp.last = q == nd - 1;
       void** dst = fp.last ? a.mu : a.kb[q % 2];
       for (int v = 0; v < V; ++v) {
         fp.in[v] = (const T*)src[v];
@@ -199,6 +202,7 @@ int adjoint_step(lee_ctx* c, double dt, const double* amps, double* gbar) {
   AdjStageParams<T> p;
   memset(&p, 0, sizeof p);
   p.nx = b.nx; p.ny = b.ny; p.nz = b.nz; p.V = V;
+  p.px = b.px;
   const Coef<T>* jm = dbl ? (const Coef<T>*)b.cd_jm : (const Coef<T>*)b.cf_jm;
   for (int q = 0; q < 9; ++q) p.jm[q] = jm[q];
   for (int x = 0; x < 3; ++x) p.ubar[x] = dbl ? (T)b.cd_ub[x].c : (T)b.cf_ub[x].c;
@@ -323,7 +327,8 @@ int lee_set_objective(lee_ctx* c, int b, int n, const long long* l0, double weig
   a.mic = mic;
   a.mic_block = b;
   a.weight = weight;
-  CK(cudaMemcpyAsync(a.d_mic, a.mic.data(), a.mic.size() * sizeof(long long), cudaMemcpyHostToDevice, c->stream));
+  for (auto& l : mic) l = row_pos(l, bk.nx, bk.px);  // as the state fields hold the points
+  CK(cudaMemcpyAsync(a.d_mic, mic.data(), mic.size() * sizeof(long long), cudaMemcpyHostToDevice, c->stream));
   if (!a.d_base) {
     int rc = dalloc(c, &a.d_base, 1);
     if (rc) return rc;
@@ -361,10 +366,10 @@ int lee_apply_adjoint(lee_ctx* c, int nsteps, double dt) {
   for (size_t bi = 0; bi < c->blk.size(); ++bi) {
     BlockData& b = c->blk[bi];
     void** lam = lam_of(c, (int)bi);
-    const size_t bytes = (size_t)b.N * c->esz;
+    const size_t bytes = (size_t)b.NP * c->esz;
     for (int v = 0; v < c->V; ++v) {
       if (c->comp) {
-        k_add_pair<<<grid1d(b.N), 256, 0, c->stream>>>(b.N, (float*)lam[v], (const float*)b.y[v],
+        k_add_pair<<<grid1d(b.NP), 256, 0, c->stream>>>(b.NP, (float*)lam[v], (const float*)b.y[v],
                                                         (const float*)b.comp[v]);
         CK(cudaGetLastError());
       } else {
@@ -383,7 +388,7 @@ int lee_apply_adjoint(lee_ctx* c, int nsteps, double dt) {
   for (size_t bi = 0; bi < c->blk.size(); ++bi) {
     BlockData& b = c->blk[bi];
     void** lam = lam_of(c, (int)bi);
-    const size_t bytes = (size_t)b.N * c->esz;
+    const size_t bytes = (size_t)b.NP * c->esz;
     for (int v = 0; v < c->V; ++v) {
       CK(cudaMemcpyAsync(b.y[v], lam[v], bytes, cudaMemcpyDeviceToDevice, c->stream));
       if (c->comp) CK(cudaMemsetAsync(b.comp[v], 0, bytes, c->stream));
@@ -435,7 +440,7 @@ int lee_adjoint_gradient(lee_ctx* c, int nsteps, double dt, int checkpoint_every
     BlockData& b = c->blk[(size_t)q.b];
     return q.kind == 0 ? b.y[q.v] : q.kind == 1 ? b.comp[q.v] : b.rho;
   };
-  auto bytes_of = [&](const Slot& q) { return (size_t)c->blk[(size_t)q.b].N * c->esz; };
+  auto bytes_of = [&](const Slot& q) { return (size_t)c->blk[(size_t)q.b].NP * c->esz; };
   const size_t fields = slots.size();
   if (a.ckpt_slots < (size_t)nseg || a.ckpt.size() < (size_t)nseg * fields) {
     for (size_t q = a.ckpt.size(); q < (size_t)nseg * fields; ++q) {
@@ -498,7 +503,7 @@ int lee_adjoint_gradient(lee_ctx* c, int nsteps, double dt, int checkpoint_every
   CK(cudaMemsetAsync(a.d_gbar, 0, nbox * sizeof(double), c->stream));
   for (int bi = 0; bi < nbk; ++bi) {
     void** lam = lam_of(c, bi);
-    for (int v = 0; v < V; ++v) CK(cudaMemsetAsync(lam[v], 0, (size_t)c->blk[(size_t)bi].N * c->esz, c->stream));
+    for (int v = 0; v < V; ++v) CK(cudaMemsetAsync(lam[v], 0, (size_t)c->blk[(size_t)bi].NP * c->esz, c->stream));
   }
   a.rb_live = false;
   const Tableau tb = tableau(c->cfg.rk_scheme);

@@ -45,23 +45,27 @@ int adjoint_gen_setup(lee_ctx* c) {
   for (int bi = 0; bi < nbk; ++bi) {
     BlockData& b = c->blk[(size_t)bi];
     auto& g = a.gb[(size_t)bi];
-    if ((rc = alloc_fields(c, g.lam, b.N)) || (rc = alloc_fields(c, g.mu, b.N)) ||
-        (rc = alloc_fields(c, g.kb[0], b.N)) || (rc = alloc_fields(c, g.kb[1], b.N)) ||
-        (rc = alloc_fields(c, g.ybar, b.N)) || (rc = alloc_fields(c, g.nu, b.N)))
+    if ((rc = alloc_fields(c, g.lam, b.NP)) || (rc = alloc_fields(c, g.mu, b.NP)) ||
+        (rc = alloc_fields(c, g.kb[0], b.NP)) || (rc = alloc_fields(c, g.kb[1], b.NP)) ||
+        (rc = alloc_fields(c, g.ybar, b.NP)) || (rc = alloc_fields(c, g.nu, b.NP)))
       return rc;
     for (int d = 0; d < c->cfg.num_dim; ++d)
-      if ((rc = alloc_fields(c, g.g[d], b.N))) return rc;
+      if ((rc = alloc_fields(c, g.g[d], b.NP))) return rc;
     if (b.need_rho)
       for (int q = 0; q < 2; ++q) {
-        if ((rc = dev_alloc(c, &g.rb[q], (size_t)b.N * c->esz))) return rc;
-        CK(cudaMemsetAsync(g.rb[q], 0, (size_t)b.N * c->esz, c->stream));
+        if ((rc = dev_alloc(c, &g.rb[q], (size_t)b.NP * c->esz))) return rc;
+        CK(cudaMemsetAsync(g.rb[q], 0, (size_t)b.NP * c->esz, c->stream));
       }
   }
   auto& o = c->ovs;
   if (o.n > 0) {
     // the receivers are distinct points (each forward value is overwritten once)
     std::vector<std::pair<int, long long>> recv((size_t)o.n);
-    for (int r = 0; r < o.n; ++r) recv[(size_t)r] = {o.rb[(size_t)r], o.rl[(size_t)r]};
+    // (points as the state fields hold them)
+    for (int r = 0; r < o.n; ++r) {
+      const BlockData& rk = c->blk[(size_t)o.rb[(size_t)r]];
+      recv[(size_t)r] = {o.rb[(size_t)r], row_pos(o.rl[(size_t)r], rk.nx, rk.px)};
+    }
     std::sort(recv.begin(), recv.end());
     for (size_t q = 1; q < recv.size(); ++q)
       if (recv[q] == recv[q - 1]) return fail(c, LEE_ERR_UNSUPPORTED, "the adjoint needs distinct overset receivers");
@@ -76,12 +80,13 @@ int adjoint_gen_setup(lee_ctx* c) {
     taps.reserve((size_t)o.n * o.W);
     for (int r = 0; r < o.n; ++r) {
       const int db = o.db[(size_t)r];
-      const long long nx = c->blk[(size_t)db].nx, nxy = nx * c->blk[(size_t)db].ny;
+      const BlockData& dk = c->blk[(size_t)db];
+      const long long nx = dk.px, nxy = nx * dk.ny, l0 = row_pos(o.dl[(size_t)r], dk.nx, dk.px);
       int st = 0;
       for (int w3 = 0; w3 < o.w[2]; ++w3)
         for (int w2 = 0; w2 < o.w[1]; ++w2)
           for (int w1 = 0; w1 < o.w[0]; ++w1)
-            taps.push_back({db, o.dl[(size_t)r] + w1 + w2 * nx + w3 * nxy, r, o.wt[(size_t)r * o.W + st++]});
+            taps.push_back({db, l0 + w1 + w2 * nx + w3 * nxy, r, o.wt[(size_t)r * o.W + st++]});
     }
     std::stable_sort(taps.begin(), taps.end(), [](const Tap& x, const Tap& y) {
       if (x.b != y.b) return x.b < y.b;
@@ -125,8 +130,8 @@ template <typename T>
 AdjGenPoint<T> point_ops(lee_ctx* c, BlockData& b) {
   AdjGenPoint<T> p;
   memset(&p, 0, sizeof p);
-  p.iblank = b.has_holes ? b.d_iblank : nullptr;
-  p.pbar = b.d_mean[4];
+  p.iblank = b.has_holes ? b.d_tiblank : nullptr;
+  p.pbar = b.d_tpbar;
   p.inv_gamma = (T)(1.0 / c->cfg.gamma);
   return p;
 }
@@ -200,15 +205,16 @@ int adjoint_step_gen(lee_ctx* c, double dt, const double* amps, double* gbar, bo
         AdjGenFilterParams<T> fp;
         memset(&fp, 0, sizeof fp);
         fp.nx = b.nx; fp.ny = b.ny; fp.nz = b.nz; fp.V = V;
+        fp.px = b.px;
         fp.dir = dirs[q];
         fp.last = q == 0;
-        fp.iblank = b.has_holes ? b.d_iblank : nullptr;
+        fp.iblank = b.has_holes ? b.d_tiblank : nullptr;
         fp.mask_in = (q == nd - 1 && fp.iblank) ? 1 : 0;
-        fp.code = b.has_holes ? b.d_code_flt[dirs[q]] : nullptr;
+        fp.code = b.has_holes ? b.d_tcode_flt[dirs[q]] : nullptr;
         fp.op = c->flt;
         fp.blend = (T)c->cfg.filter_blend;
         fp.rb = fp.last ? rb : nullptr;
-        fp.pbar = b.d_mean[4];
+        fp.pbar = b.d_tpbar;
         fp.inv_gamma = (T)(1.0 / c->cfg.gamma);
         void** dst = fp.last ? g.mu : g.kb[q % 2];
         for (int v = 0; v < V; ++v) {
@@ -227,7 +233,7 @@ int adjoint_step_gen(lee_ctx* c, double dt, const double* amps, double* gbar, bo
         p.in[v] = (const T*)g.lam[v];
         p.out[v] = (T*)g.mu[v];
       }
-      CK(launch_adjg_mask<T>(b.N, V, p, c->stream));
+      CK(launch_adjg_mask<T>(b.NP, V, p, c->stream));
       c->stats.kernel_launches += 1;
     }
   }
@@ -243,11 +249,11 @@ int adjoint_step_gen(lee_ctx* c, double dt, const double* amps, double* gbar, bo
         p.in[v] = (const T*)g.mu[v];
         p.out[v] = (T*)g.mu[v];
       }
-      CK(launch_adjg_mask<T>(b.N, V, p, c->stream));
+      CK(launch_adjg_mask<T>(b.NP, V, p, c->stream));
       c->stats.kernel_launches += 1;
     }
     for (int v = 0; v < V; ++v)
-      CK(cudaMemcpyAsync(g.ybar[v], g.mu[v], (size_t)b.N * c->esz, cudaMemcpyDeviceToDevice, c->stream));
+      CK(cudaMemcpyAsync(g.ybar[v], g.mu[v], (size_t)b.NP * c->esz, cudaMemcpyDeviceToDevice, c->stream));
   }
   // the stages, last to first: kbar_{S-1} = h b_{S-1} mu (as the scale of mu), then
   // zbar_s = L_s^T kbar_s, nu_s = M P^T zbar_s, kbar_{s-1} = h b_{s-1} mu + a_{s-1} h nu_s
@@ -289,7 +295,7 @@ int adjoint_step_gen(lee_ctx* c, double dt, const double* amps, double* gbar, bo
       }
       const double hb = s > 0 ? dt * tb.b[s - 1] : 0.0;
       const double ha = s > 0 ? tb.a[s - 1] * dt : 0.0;
-      CK(launch_adjg_combine<T>(b.N, V, p, hb, ha, c->stream));
+      CK(launch_adjg_combine<T>(b.NP, V, p, hb, ha, c->stream));
       c->stats.kernel_launches += 1;
     }
     cur = top ? 0 : 1 - cur;

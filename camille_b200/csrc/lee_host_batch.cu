@@ -102,6 +102,7 @@ std::vector<BatchFilterInst<T>> batch_filter_inst(lee_ctx* c, bool scratch) {
     BatchFilterInst<T> f;
     memset(&f, 0, sizeof f);
     f.nx = b.nx;
+    f.px = b.px;
     f.ny = b.ny;
     void** last_out = b.zb[(tb.ns - 1) % 2];
     void** other = b.zb[tb.ns % 2];

@@ -9,9 +9,9 @@ using namespace lee;
 namespace {
 
 template <typename T>
-__global__ void k_convert(long long n, T* out, const double* in) {
+__global__ void k_convert(long long n, int nx, int px, T* out, const double* in) {
   for (long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x; l < n; l += (long long)gridDim.x * blockDim.x)
-    out[l] = (T)in[l];
+    out[row_pos(l, nx, px)] = (T)in[l];
 }
 
 // flag = 1 when some element of the fields is not finite (vector loads: the fields are
@@ -40,9 +40,11 @@ __global__ void k_nonfinite(long long n, int nf, const T* f0, const T* f1, const
 }
 
 template <typename T>
-__global__ void k_to_double(long long n, double* out, const T* y, const T* comp) {
-  for (long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x; l < n; l += (long long)gridDim.x * blockDim.x)
-    out[l] = comp ? (double)y[l] + (double)comp[l] : (double)y[l];
+__global__ void k_to_double(long long n, int nx, int px, double* out, const T* y, const T* comp) {
+  for (long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x; l < n; l += (long long)gridDim.x * blockDim.x) {
+    const long long q = row_pos(l, nx, px);
+    out[l] = comp ? (double)y[q] + (double)comp[q] : (double)y[q];
+  }
 }
 
 }  // namespace
@@ -272,13 +274,14 @@ int make_coef(lee_ctx* c, BlockData& b, const double* d_field, double scale, Coe
     return LEE_OK;
   }
   b.n_coef_fields += 1;
-  if (std::is_same<T, double>::value) {
+  if (std::is_same<T, double>::value && b.px == b.nx) {
     out->p = reinterpret_cast<const T*>(d_field);
   } else {
     T* d = nullptr;
-    rc = dalloc(c, &d, (size_t)b.N);
+    rc = dalloc(c, &d, (size_t)b.NP);
     if (rc) return rc;
-    launch_convert<T>(c->stream, b.N, d, d_field);
+    if (b.px != b.nx) CK(cudaMemsetAsync(d, 0, (size_t)b.NP * sizeof(T), c->stream));
+    launch_convert<T>(c->stream, b.N, d, d_field, b.nx, b.px);
     CK(cudaGetLastError());
     out->p = d;
   }
@@ -309,6 +312,7 @@ template <typename T>
 void fill_stage_common(lee_ctx* c, BlockData& b, StageParams<T>& p) {
   memset(&p, 0, sizeof p);
   p.nx = b.nx; p.ny = b.ny; p.nz = b.nz;
+  p.px = b.px;
   p.dim = c->cfg.num_dim;
   p.V = c->V;
   const bool dbl = std::is_same<T, double>::value;
@@ -337,8 +341,8 @@ void fill_stage_common(lee_ctx* c, BlockData& b, StageParams<T>& p) {
   p.has_src = b.d_src_g != nullptr;
   for (int d = 0; d < 3; ++d) { p.src_lo[d] = b.src_lo[d]; p.src_hi[d] = b.src_hi[d]; }
   p.src_g = dbl ? (const T*)b.d_src_g : (const T*)b.d_src_g_t;
-  for (int d = 0; d < 3; ++d) p.code[d] = b.has_holes ? b.d_code_fd[d] : nullptr;
-  p.iblank = b.has_holes ? b.d_iblank : nullptr;
+  for (int d = 0; d < 3; ++d) p.code[d] = b.has_holes ? b.d_tcode_fd[d] : nullptr;
+  p.iblank = b.has_holes ? b.d_tiblank : nullptr;
   p.fd = c->fd;
   p.sigma = (const T*)b.d_sigma_field;
 }
@@ -514,17 +518,17 @@ template void fill_stage_common<double>(lee_ctx* c, BlockData& b, StageParams<do
 
 // Launches of the conversion kernels for the other host translation units.
 template <typename T>
-void launch_convert(cudaStream_t s, long long n, T* out, const double* in) {
-  k_convert<T><<<grid1d(n), 256, 0, s>>>(n, out, in);
+void launch_convert(cudaStream_t s, long long n, T* out, const double* in, int nx, int px) {
+  k_convert<T><<<grid1d(n), 256, 0, s>>>(n, nx, px, out, in);
 }
 template <typename T>
-void launch_to_double(cudaStream_t s, long long n, double* out, const T* y, const T* comp) {
-  k_to_double<T><<<grid1d(n), 256, 0, s>>>(n, out, y, comp);
+void launch_to_double(cudaStream_t s, long long n, double* out, const T* y, const T* comp, int nx, int px) {
+  k_to_double<T><<<grid1d(n), 256, 0, s>>>(n, nx, px, out, y, comp);
 }
-template void launch_convert<float>(cudaStream_t, long long, float*, const double*);
-template void launch_convert<double>(cudaStream_t, long long, double*, const double*);
-template void launch_to_double<float>(cudaStream_t, long long, double*, const float*, const float*);
-template void launch_to_double<double>(cudaStream_t, long long, double*, const double*, const double*);
+template void launch_convert<float>(cudaStream_t, long long, float*, const double*, int, int);
+template void launch_convert<double>(cudaStream_t, long long, double*, const double*, int, int);
+template void launch_to_double<float>(cudaStream_t, long long, double*, const float*, const float*, int, int);
+template void launch_to_double<double>(cudaStream_t, long long, double*, const double*, const double*, int, int);
 
 cudaError_t launch_nonfinite(cudaStream_t s, long long n, int V, size_t esz, void* const* f, void* const* e,
                              int* flag) {

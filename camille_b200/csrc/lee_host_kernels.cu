@@ -26,13 +26,14 @@ int run_filter(lee_ctx* c, BlockData& b, void** in, void** err, void** comp_out,
     FilterParams<T> fp;
     memset(&fp, 0, sizeof fp);
     fp.nx = b.nx; fp.ny = b.ny; fp.nz = b.nz;
+    fp.px = b.px;
     fp.V = c->V;
     fp.dir = passes[q];
     fp.first = q == 0;
     fp.last = q == np - 1;
     fp.blend = (T)c->cfg.filter_blend;
-    fp.code = b.has_holes ? b.d_code_flt[passes[q]] : nullptr;
-    fp.iblank = b.has_holes ? b.d_iblank : nullptr;
+    fp.code = b.has_holes ? b.d_tcode_flt[passes[q]] : nullptr;
+    fp.iblank = b.has_holes ? b.d_tiblank : nullptr;
     fp.op = c->comp ? c->fltd : c->flt;
     void** dst = fr[q % 2];
     for (int v = 0; v < c->V; ++v) {
@@ -82,7 +83,7 @@ int encode_maps(lee_ctx* c, const BlockData& b, const void* const* fields, int n
     if (it == c->tmaps.end()) {
       CUtensorMap m;
       cuuint64_t dims[3] = {(cuuint64_t)b.nx, (cuuint64_t)b.ny, (cuuint64_t)b.nz};
-      cuuint64_t strides[2] = {(cuuint64_t)b.nx * c->esz, (cuuint64_t)b.nx * b.ny * c->esz};
+      cuuint64_t strides[2] = {(cuuint64_t)b.px * c->esz, (cuuint64_t)b.px * b.ny * c->esz};
       cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, 1};
       cuuint32_t es[3] = {1, 1, 1};
       CUresult r = c->encode(&m, c->esz == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
@@ -175,7 +176,7 @@ int launch_stage_any(lee_ctx* c, BlockData& b, const StageParams<T>& p, void* co
                                   : (p.last ? (p.increment ? kKindLastIncrement : kKindLast) : kKindMid);
   const int tr = b.traits | (kind << kKindShift);
   if constexpr (sizeof(T) == 4) {
-    if (b.stage_px == 2 && stage_pair_applies(tr, b.nx)) {
+    if (b.stage_px == 2 && stage_pair_applies(tr, b.px)) {
       CK(launch_stage_pair(fm, tp, tr, b.tiles_x * b.tiles_y, chunks, c->stream));
       return LEE_OK;
     }
@@ -191,6 +192,7 @@ int launch_filter_fused(lee_ctx* c, BlockData& b, void* const* in, void* const* 
   TmaFilterParams<T> fp;
   memset(&fp, 0, sizeof fp);
   fp.nx = b.nx; fp.ny = b.ny; fp.nz = b.nz;
+  fp.px = b.px;
   fp.V = c->V;
   fp.tiles_x = b.tiles_x;
   fp.k_chunk = chunk_override ? chunk_override : b.filter_chunk;
@@ -198,8 +200,8 @@ int launch_filter_fused(lee_ctx* c, BlockData& b, void* const* in, void* const* 
   for (int a = 0; a < 12; ++a)
     for (int o = 0; o < 11; ++o) fp.w[a][o] = (T)c->wfl[a][o];
   if (b.has_holes) {
-    for (int d = 0; d < 3; ++d) fp.code[d] = b.d_code_flt[d];
-    fp.iblank = b.d_iblank;
+    for (int d = 0; d < 3; ++d) fp.code[d] = b.d_tcode_flt[d];
+    fp.iblank = b.d_tiblank;
   }
   fp.blend = (T)c->cfg.filter_blend;
   for (int v = 0; v < c->V; ++v) {
@@ -262,9 +264,13 @@ int autotune(lee_ctx* c, BlockData& b) {
   // plane chunks: a fixed ladder (stage kernels), and for the filter also the near-equal splits
   // of the block's planes into 1..24 chunks (ceil(nz / c): every chunk but the last of the same
   // length, so that CTA counts that fill whole waves of the GPU are among the candidates)
-  const std::vector<int> ladder = {8, 16, 24, 32, 48, 64, 96, 128, 192, 256};
-  std::vector<int> splits = ladder;
-  for (int q = 1; q <= 24; ++q) splits.push_back((b.nz + q - 1) / q);
+  std::vector<int> ladder = {8, 16, 24, 32, 48, 64, 96, 128, 192, 256};
+  if (b.nz < ladder[0]) ladder.push_back(b.nz);
+  std::vector<int> splits;
+  for (int q = 1; q <= 24; ++q) {
+    const int ch = (b.nz + q - 1) / q;
+    if (std::find(ladder.begin(), ladder.end(), ch) == ladder.end()) splits.push_back(ch);
+  }
   std::sort(splits.begin(), splits.end());
   splits.erase(std::unique(splits.begin(), splits.end()), splits.end());
   const std::vector<int> cands2 = {1};
@@ -289,67 +295,74 @@ int autotune(lee_ctx* c, BlockData& b) {
     int best_scalar_chunk = b.nz, best_scalar_ry = b.filter_ry;
     // the scalar filter's forms (1: one tile row per thread row, 2: two rows, 3: two points per
     // thread) are timed with the chunk: each point's arithmetic is the same in all three
-    const int nry = which == 1 && c->filter_form == 0 ? 3 : 1;
-    for (int kq = 0; kq < (which == 1 ? nkinds : nskinds) * nry; ++kq) {
-      if (which == 0) {
-        b.stage_px = skinds[kq];
-      } else {
-        b.filter_px = kinds[kq / nry];
-        const int form = c->filter_form > 0 ? c->filter_form : 1 + kq % nry;
-        // the one-row form alone takes holes and the increment step's input (a form set by
-        // lee_set_filter_form is kept, and the increment step then does not apply)
-        if (c->filter_form == 0 && (b.filter_px > 0 || b.has_holes || (c->comp && c->increment_step)) && form > 1)
-          continue;
-        if (form == 3 && !b.filter_pair_ok) continue;
-        b.filter_ry = form == 2 ? 2 : 1;
-        b.filter_pair = form == 3;
-        set_filter_tiles(c, b);
-      }
-      for (int ch : (d3 ? (which == 1 ? splits : ladder) : cands2)) {
-        if (d3 && ch > b.nz) continue;
-        float tsum = 0.f;
-        for (int rep = 0; rep < 4; ++rep) {  // the first run warms up
-          CK(cudaEventRecord(e0, c->stream));
-          int rc;
-          if (which == 0) {
-            StageParams<T> p;
-            fill_stage_common<T>(c, b, p);
-            p.stage = 1;
-            p.last = 0;
-            p.h = (T)1e-3;
-            p.b = (T)(1.0 / 3.0);
-            p.a = (T)0.5;
-            for (int v = 0; v < c->V; ++v) {
-              p.zin[v] = (const T*)b.zb[0][v];
-              p.yn[v] = (const T*)b.y[v];
-              p.acc[v] = (T*)b.acc[v];
-              p.zout[v] = (T*)b.zb[1][v];
-              p.comp[v] = (T*)b.comp[v];
+    const int nry = which == 1 && b.filter_form == 0 ? 3 : 1;
+    // the ladder for every form, then the filter's other splits for the form that won there (a
+    // third of the launches of every split for every form: 12 instead of 40 ms at 129 x 113 x 97)
+    int best_kq = 0;
+    for (int phase = 0; phase < (d3 && which == 1 ? 2 : 1); ++phase) {
+      for (int kq = 0; kq < (which == 1 ? nkinds : nskinds) * nry; ++kq) {
+        if (phase == 1 && kq != best_kq) continue;
+        if (which == 0) {
+          b.stage_px = skinds[kq];
+        } else {
+          b.filter_px = kinds[kq / nry];
+          const int form = b.filter_form > 0 ? b.filter_form : 1 + kq % nry;
+          // the one-row form alone takes holes and the increment step's input (a form set by
+          // lee_set_filter_form is kept, and the increment step then does not apply)
+          if (b.filter_form == 0 && (b.filter_px > 0 || b.has_holes || (c->comp && c->increment_step)) && form > 1)
+            continue;
+          if (form == 3 && !b.filter_pair_ok) continue;
+          b.filter_ry = form == 2 ? 2 : 1;
+          b.filter_pair = form == 3;
+          set_filter_tiles(c, b);
+        }
+        for (int ch : (d3 ? (phase == 1 ? splits : ladder) : cands2)) {
+          if (d3 && ch > b.nz) continue;
+          float tsum = 0.f;
+          for (int rep = 0; rep < 3; ++rep) {  // the first run warms up
+            CK(cudaEventRecord(e0, c->stream));
+            int rc;
+            if (which == 0) {
+              StageParams<T> p;
+              fill_stage_common<T>(c, b, p);
+              p.stage = 1;
+              p.last = 0;
+              p.h = (T)1e-3;
+              p.b = (T)(1.0 / 3.0);
+              p.a = (T)0.5;
+              for (int v = 0; v < c->V; ++v) {
+                p.zin[v] = (const T*)b.zb[0][v];
+                p.yn[v] = (const T*)b.y[v];
+                p.acc[v] = (T*)b.acc[v];
+                p.zout[v] = (T*)b.zb[1][v];
+                p.comp[v] = (T*)b.comp[v];
+              }
+              rc = launch_stage_any<T>(c, b, p, b.zb[0], d3 ? ch : 0);
+            } else {
+              const int chunk = d3 ? ch : 0;
+              rc = c->comp ? launch_filter_fused<T>(c, b, b.zb[1], b.acc, b.zb[0], b.comp, chunk)
+                           : launch_filter_fused<T>(c, b, b.acc, nullptr, b.zb[0], nullptr, chunk);
             }
-            rc = launch_stage_any<T>(c, b, p, b.zb[0], d3 ? ch : 0);
-          } else {
-            const int chunk = d3 ? ch : 0;
-            rc = c->comp ? launch_filter_fused<T>(c, b, b.zb[1], b.acc, b.zb[0], b.comp, chunk)
-                         : launch_filter_fused<T>(c, b, b.acc, nullptr, b.zb[0], nullptr, chunk);
+            if (rc) return rc;
+            CK(cudaEventRecord(e1, c->stream));
+            CK(cudaEventSynchronize(e1));
+            float ms = 0.f;
+            CK(cudaEventElapsedTime(&ms, e0, e1));
+            if (rep > 0) tsum += ms;
           }
-          if (rc) return rc;
-          CK(cudaEventRecord(e1, c->stream));
-          CK(cudaEventSynchronize(e1));
-          float ms = 0.f;
-          CK(cudaEventElapsedTime(&ms, e0, e1));
-          if (rep > 0) tsum += ms;
-        }
-        if (which == 1 && !b.filter_pair && tsum < best_scalar) {
-          best_scalar = tsum;
-          best_scalar_chunk = d3 ? ch : b.nz;
-          best_scalar_ry = b.filter_ry;
-        }
-        if (tsum < best) {
-          best = tsum;
-          best_chunk = d3 ? ch : b.nz;
-          best_kind = which == 0 ? b.stage_px : b.filter_px;
-          best_ry = b.filter_ry;
-          best_pair = b.filter_pair;
+          if (which == 1 && !b.filter_pair && tsum < best_scalar) {
+            best_scalar = tsum;
+            best_scalar_chunk = d3 ? ch : b.nz;
+            best_scalar_ry = b.filter_ry;
+          }
+          if (tsum < best) {
+            best = tsum;
+            best_kq = kq;
+            best_chunk = d3 ? ch : b.nz;
+            best_kind = which == 0 ? b.stage_px : b.filter_px;
+            best_ry = b.filter_ry;
+            best_pair = b.filter_pair;
+          }
         }
       }
     }
@@ -389,7 +402,7 @@ int check_device_error(lee_ctx* c) {
 // The non-finite sentinel: every value of the state is checked (the carried rounding error of
 // the compensated form follows the state); any NaN or infinity sets d_err[1].
 int check_finite(lee_ctx* c) {
-  for (auto& b : c->blk) CK(launch_nonfinite(c->stream, b.N, c->V, c->esz, b.y, nullptr, c->d_err + 1));
+  for (auto& b : c->blk) CK(launch_nonfinite(c->stream, b.NP, c->V, c->esz, b.y, nullptr, c->d_err + 1));
   return LEE_OK;
 }
 
@@ -407,7 +420,8 @@ void fill_bc_params(lee_ctx* c, const BlockData& b, const Boundary& z, void** f,
   p.lo[z.dir] = z.end == 0 ? z.lo[z.dir] : z.hi[z.dir];
   p.nb[z.dir] = 1;
   p.nx = b.nx; p.ny = b.ny;
-  p.sd = z.dir == 0 ? 1 : z.dir == 1 ? (long long)b.nx : (long long)b.nx * b.ny;
+  p.px = b.px;
+  p.sd = z.dir == 0 ? 1 : z.dir == 1 ? (long long)b.px : (long long)b.px * b.ny;
   p.S = c->fd.S;
   for (int q = 0; q < c->fd.S; ++q) p.c0[q] = c->fd.B[0][q];
   for (int v = 0; v < c->V; ++v) {

@@ -170,6 +170,15 @@ int lee_get_overset(lee_ctx* c, int* recv_block, long long* recv_l0, int* donor_
   if (donor_l0) CK(cudaMemcpyAsync(donor_l0, o.d_dl, n * sizeof(long long), cudaMemcpyDeviceToHost, c->stream));
   if (weights) CK(cudaMemcpyAsync(weights, o.d_wt, n * o.W * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
+  // back from the state fields' rows to the caller's
+  auto user = [&](long long& l, int b) {
+    const BlockData& bk = c->blk[(size_t)b];
+    l = (l / bk.px) * bk.nx + l % bk.px;
+  };
+  for (size_t r = 0; r < n; ++r) {
+    if (recv_l0) user(recv_l0[r], o.rb[r]);
+    if (donor_l0) user(donor_l0[r], o.db[r]);
+  }
   return LEE_OK;
 }
 

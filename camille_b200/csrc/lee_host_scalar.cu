@@ -189,7 +189,7 @@ int scalar_overset(lee_ctx* c, int s, int ns) {
         op.y[bi][v] = (T*)f[k0 + v];
         op.e[bi][v] = (T*)e[k0 + v];
       }
-      op.nx[bi] = b.nx;
+      op.px[bi] = b.px;
       op.ny[bi] = b.ny;
     }
     CK(launch_overset<T>(op, c->stream));
@@ -223,6 +223,7 @@ int scalar_filter(lee_ctx* c, BlockData& b, int ns) {
       FilterParams<T> fp;
       memset(&fp, 0, sizeof fp);
       fp.nx = b.nx; fp.ny = b.ny; fp.nz = b.nz;
+      fp.px = b.px;
       fp.V = nk;
       fp.dir = passes[q];
       fp.first = q == 0;

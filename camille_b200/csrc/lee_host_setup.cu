@@ -8,12 +8,18 @@ using namespace lee;
 
 namespace {
 
-__global__ void k_add_box(int nx, int ny, int lo0, int lo1, int lo2, int b0, int b1, long long nb, const double* sig,
+__global__ void k_add_box(int px, int ny, int lo0, int lo1, int lo2, int b0, int b1, long long nb, const double* sig,
                           double* field) {
   for (long long lb = blockIdx.x * (long long)blockDim.x + threadIdx.x; lb < nb; lb += (long long)gridDim.x * blockDim.x) {
     const int i = lo0 + (int)(lb % b0), j = lo1 + (int)((lb / b0) % b1), k = lo2 + (int)(lb / ((long long)b0 * b1));
-    field[i + (long long)nx * (j + (long long)ny * k)] += sig[lb];
+    field[i + (long long)px * (j + (long long)ny * k)] += sig[lb];
   }
+}
+
+template <typename P>
+__global__ void k_at_pitch(long long n, int nx, int px, P* out, const P* in) {
+  for (long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x; l < n; l += (long long)gridDim.x * blockDim.x)
+    out[row_pos(l, nx, px)] = in[l];
 }
 
 template <typename T>
@@ -22,9 +28,38 @@ __global__ void k_fill_const(long long n, T* out, T v) {
     out[l] = v;
 }
 
+// A setup field at the time loop's row pitch, pads `fill` (the field itself when px = nx).
+template <typename P>
+int at_pitch(lee_ctx* c, const BlockData& b, P* in, P fill, P** out) {
+  *out = in;
+  if (b.px == b.nx) return LEE_OK;
+  int rc = dalloc(c, out, (size_t)b.NP);
+  if (rc) return rc;
+  k_fill_const<P><<<grid1d(b.NP), 256, 0, c->stream>>>(b.NP, *out, fill);
+  k_at_pitch<P><<<grid1d(b.N), 256, 0, c->stream>>>(b.N, b.nx, b.px, *out, in);
+  CK(cudaGetLastError());
+  return LEE_OK;
+}
+
 }  // namespace
 
 namespace lee {
+
+// The row pitch of a block's time-loop arrays: nx, or where nx values are no whole number of 16
+// bytes and the TMA-staged stage or filter kernel would run but for that (a tensor map's rows
+// start on 16 bytes), nx rounded up to one. At 129 x 113 x 97 in FP32 the step went from 1.11 to
+// 0.32 ms (generic kernels: one load per tap through L1; at most 3 points per row of padding).
+// Passive scalars and axisymmetric contexts, which run the generic kernels, stay unpadded.
+void set_pitch(const lee_ctx* c, BlockData& b) {
+  b.px = b.nx;
+  bool wave_zone = false;
+  for (auto& z : b.bnd) wave_zone |= z.kind == LEE_SPONGE_FREUND_HARMONICWAVE;
+  const bool stage = c->wst_ok && !wave_zone;
+  const bool filter = c->wfl_ok && c->cfg.filter_scheme != LEE_FILTER_NONE && (!b.has_holes || 1 + 2 * c->flt.nb < 12);
+  const int a = (int)(16 / c->esz);
+  if (c->nsc == 0 && !c->axisym && (stage || filter)) b.px = (b.nx + a - 1) / a * a;
+  b.NP = (long long)b.px * b.ny * b.nz;
+}
 
 // metrics::compute with Thomas-Lombard products (src/metrics/metrics.cpp:9-251), the
 // Jacobian (:255-328; 3-D determinant of oracle patch P1) and inverse metrics (:355-426).
@@ -106,14 +141,14 @@ int compute_metrics(lee_ctx* c, BlockData& b) {
 // precision of the stage kernels.
 int build_sigma_field(lee_ctx* c, BlockData& b) {
   double* f = nullptr;
-  int rc = dalloc(c, &f, (size_t)b.N);
+  int rc = dalloc(c, &f, (size_t)b.NP);
   if (rc) return rc;
-  CK(cudaMemsetAsync(f, 0, (size_t)b.N * 8, c->stream));
+  CK(cudaMemsetAsync(f, 0, (size_t)b.NP * 8, c->stream));
   for (auto& z : b.bnd) {
     if (!is_sponge(z.kind)) continue;
     const int b0 = z.hi[0] - z.lo[0] + 1, b1 = z.hi[1] - z.lo[1] + 1, b2 = z.hi[2] - z.lo[2] + 1;
     const long long nb = (long long)b0 * b1 * b2;
-    k_add_box<<<grid1d(nb), 256, 0, c->stream>>>(b.nx, b.ny, z.lo[0], z.lo[1], z.lo[2], b0, b1, nb, z.d_sigma, f);
+    k_add_box<<<grid1d(nb), 256, 0, c->stream>>>(b.px, b.ny, z.lo[0], z.lo[1], z.lo[2], b0, b1, nb, z.d_sigma, f);
     CK(cudaGetLastError());
   }
   if (!c->comp) {
@@ -121,8 +156,8 @@ int build_sigma_field(lee_ctx* c, BlockData& b) {
     return LEE_OK;
   }
   float* g = nullptr;
-  if ((rc = dalloc(c, &g, (size_t)b.N))) return rc;
-  launch_convert<float>(c->stream, b.N, g, f);
+  if ((rc = dalloc(c, &g, (size_t)b.NP))) return rc;
+  launch_convert<float>(c->stream, b.NP, g, f);
   CK(cudaGetLastError());
   b.d_sigma_field = g;
   return LEE_OK;
@@ -148,6 +183,7 @@ int lee_prepare(lee_ctx* c) {
   for (auto& b : c->blk) {
     if (!b.set || !b.has_mean) return fail(c, LEE_ERR_STATE, "every block needs lee_set_block and lee_set_mean");
     const int N = (int)b.N;
+    set_pitch(c, b);
     if ((rc = upload(c, &b.d_xyz[0], b.hx))) return rc;
     if ((rc = upload(c, &b.d_xyz[1], b.hy))) return rc;
     if ((rc = upload(c, &b.d_xyz[2], b.hz))) return rc;
@@ -158,7 +194,9 @@ int lee_prepare(lee_ctx* c) {
       if ((rc = dalloc(c, &b.d_iblank, (size_t)N))) return rc;
       CK(cudaMemcpyAsync(b.d_iblank, b.hib.data(), (size_t)N * sizeof(int), cudaMemcpyHostToDevice, s));
       CK(cudaStreamSynchronize(s));
+      if ((rc = at_pitch(c, b, b.d_iblank, 0, &b.d_tiblank))) return rc;
     }
+    if ((rc = at_pitch(c, b, b.d_mean[4], 1.0, &b.d_tpbar))) return rc;
     // hole closures (receivers alone leave every closure as it is)
     if (b.has_holes) {
       std::vector<int8_t> code;
@@ -169,12 +207,14 @@ int lee_prepare(lee_ctx* c) {
         if ((rc = dalloc(c, &b.d_code_fd[d], (size_t)N))) return rc;
         CK(cudaMemcpyAsync(b.d_code_fd[d], code.data(), (size_t)N, cudaMemcpyHostToDevice, s));
         CK(cudaStreamSynchronize(s));
+        if ((rc = at_pitch(c, b, b.d_code_fd[d], (int8_t)0, &b.d_tcode_fd[d]))) return rc;
         if (c->cfg.filter_scheme != LEE_FILTER_NONE) {
           if (!closure_codes(c->flt, b, d, code))
             return fail(c, LEE_ERR_ARG, "filter hole closure lacks fluid support");
           if ((rc = dalloc(c, &b.d_code_flt[d], (size_t)N))) return rc;
           CK(cudaMemcpyAsync(b.d_code_flt[d], code.data(), (size_t)N, cudaMemcpyHostToDevice, s));
           CK(cudaStreamSynchronize(s));
+          if ((rc = at_pitch(c, b, b.d_code_flt[d], (int8_t)0, &b.d_tcode_flt[d]))) return rc;
         }
       }
     }
@@ -362,30 +402,30 @@ int lee_prepare(lee_ctx* c) {
     }
     b.need_rho = 0;
     for (int q = 0; q < 9; ++q) b.need_rho |= c->comp ? !b.cf_gu[q].zero : !b.cd_gu[q].zero;
-    if (b.need_rho && (rc = dev_alloc(c, &b.rho, (size_t)b.N * c->esz))) return rc;
+    if (b.need_rho && (rc = dev_alloc(c, &b.rho, (size_t)b.NP * c->esz))) return rc;
     b.rho_valid = false;
     if ((rc = scalar_setup(c, b))) return rc;
     // state buffers
-    if ((rc = alloc_fields(c, b.y, b.N))) return rc;
-    if ((rc = alloc_fields(c, b.acc, b.N))) return rc;
-    if ((rc = alloc_fields(c, b.zb[0], b.N))) return rc;
-    if ((rc = alloc_fields(c, b.zb[1], b.N))) return rc;
+    if ((rc = alloc_fields(c, b.y, b.NP))) return rc;
+    if ((rc = alloc_fields(c, b.acc, b.NP))) return rc;
+    if ((rc = alloc_fields(c, b.zb[0], b.NP))) return rc;
+    if ((rc = alloc_fields(c, b.zb[1], b.NP))) return rc;
     if (c->comp) {
-      if ((rc = alloc_fields(c, b.comp, b.N))) return rc;
-      if ((rc = alloc_fields(c, b.dsum, b.N))) return rc;
+      if ((rc = alloc_fields(c, b.comp, b.NP))) return rc;
+      if ((rc = alloc_fields(c, b.dsum, b.NP))) return rc;
     }
     // TMA-staged kernels: the 4th-order difference, rows of 16-byte multiples; on a block with
     // holes the classes come from the closure codes (one-point stage kernel, one-row filter)
-    const bool rows16 = ((size_t)b.nx * c->esz) % 16 == 0;
+    const bool rows16 = ((size_t)b.px * c->esz) % 16 == 0;
     b.tiles_x = (b.nx + kTileX - 1) / kTileX;
     b.tiles_y = (b.ny + kTileY - 1) / kTileY;
     // (the TMA stage kernel addresses points with 32-bit offsets)
     // (and the harmonic-wave sponge, an RHS term of the generic kernel's zone loop, is absent)
     bool wave_zone = false;
     for (auto& z : b.bnd) wave_zone |= z.kind == LEE_SPONGE_FREUND_HARMONICWAVE;
-    b.tma = c->wst_ok && rows16 && (unsigned long long)b.N < (1ull << 32) && !wave_zone && !c->axisym;
+    b.tma = c->wst_ok && rows16 && (unsigned long long)b.NP < (1ull << 32) && !wave_zone && !c->axisym;
     b.tma_filter = c->wfl_ok && rows16 && c->cfg.filter_scheme != LEE_FILTER_NONE &&
-                   (unsigned long long)b.N < (1ull << 32) && (!b.has_holes || 1 + 2 * c->flt.nb < 12);
+                   (unsigned long long)b.NP < (1ull << 32) && (!b.has_holes || 1 + 2 * c->flt.nb < 12);
     // the kernels are a fixed choice (they round differently, and two contexts of one case give
     // the same bits): the scalar fused filter unless another is asked for
     b.filter_vec = b.tma_filter && c->wfl_sym && !b.has_holes;
@@ -395,23 +435,27 @@ int lee_prepare(lee_ctx* c) {
       const int n = filter_vec_widths(c->esz, px);
       bool ok = c->filter_kernel == 0;
       for (int q = 0; q < n; ++q) ok |= b.filter_vec && c->filter_kernel == px[q];
-      if (!ok)
+      if (!ok && b.px == b.nx)
         return fail(c, LEE_ERR_UNSUPPORTED, "filter kernel %d is not available for block %d", c->filter_kernel,
                     (int)(&b - c->blk.data()));
-      b.filter_px = c->filter_kernel;
+      if (ok) b.filter_px = c->filter_kernel;
     }
     b.filter_ry = 1;
     // the two-point form: compensated FP32, 3-D, no holes, even nxi, the scalar kernel's place
-    b.filter_pair_ok = b.tma_filter && c->comp && c->cfg.num_dim == 3 && !b.has_holes && b.nx % 2 == 0 &&
+    b.filter_pair_ok = b.tma_filter && c->comp && c->cfg.num_dim == 3 && !b.has_holes && b.px % 2 == 0 &&
                        b.filter_px == 0 && filter_pair_half_width(c->hf);
     b.filter_pair = false;
+    b.filter_form = 0;
     if (c->filter_form > 0 && b.tma_filter) {
       // the two-row and two-point forms take neither holes nor the vector kernel's groups
-      if ((c->filter_form == 2 && (b.filter_px > 0 || b.has_holes)) || (c->filter_form == 3 && !b.filter_pair_ok))
+      const bool ok = c->filter_form == 1 || (c->filter_form == 2 && b.filter_px == 0 && !b.has_holes) ||
+                      (c->filter_form == 3 && b.filter_pair_ok);
+      if (!ok && b.px == b.nx)
         return fail(c, LEE_ERR_UNSUPPORTED, "filter form %d is not available for block %d", c->filter_form,
                     (int)(&b - c->blk.data()));
-      b.filter_ry = c->filter_form == 2 ? 2 : 1;
-      b.filter_pair = c->filter_form == 3;
+      b.filter_form = ok ? c->filter_form : 0;  // (a padded block without the choice runs its default)
+      b.filter_ry = b.filter_form == 2 ? 2 : 1;
+      b.filter_pair = b.filter_form == 3;
     }
     b.tfilter_ry = b.filter_ry;
     b.tfilter_chunk = 0;
@@ -430,13 +474,14 @@ int lee_prepare(lee_ctx* c) {
       uni &= is_const(b.cd_pb, b.cf_pb) && is_const(b.cd_rbi, b.cf_rbi) && !b.need_rho;
       for (auto& z : b.bnd) spg |= is_sponge(z.kind);
       b.traits = kTrTma | (jmf ? kTrJmField : 0) | (uni ? kTrUniform : 0) | (spg ? kTrSponge : 0);
-      b.stage_pair = c->comp && uni && b.nx % 2 == 0 && !b.has_holes;
+      b.stage_pair = c->comp && uni && b.px % 2 == 0 && !b.has_holes;
       b.stage_px = b.stage_pair ? 2 : 1;
       if (c->stage_kernel > 0) {
-        if (c->stage_kernel != 1 && !(c->stage_kernel == 2 && b.stage_pair))
+        const bool ok = c->stage_kernel == 1 || (c->stage_kernel == 2 && b.stage_pair);
+        if (!ok && b.px == b.nx)
           return fail(c, LEE_ERR_UNSUPPORTED, "stage kernel %d is not available for block %d", c->stage_kernel,
                       (int)(&b - c->blk.data()));
-        b.stage_px = c->stage_kernel;
+        if (ok) b.stage_px = c->stage_kernel;  // (a padded block without the choice runs its default)
       }
       if (spg && (rc = build_sigma_field(c, b))) return rc;
       if (jmf) {
@@ -447,14 +492,14 @@ int lee_prepare(lee_ctx* c) {
             const int q = l * 3 + x;
             if (c->comp && !b.cf_jm[q].p) {
               float* f = nullptr;
-              if ((rc = dalloc(c, &f, (size_t)b.N))) return rc;
-              k_fill_const<float><<<grid1d(b.N), 256, 0, c->stream>>>(b.N, f, b.cf_jm[q].c);
+              if ((rc = dalloc(c, &f, (size_t)b.NP))) return rc;
+              k_fill_const<float><<<grid1d(b.NP), 256, 0, c->stream>>>(b.NP, f, b.cf_jm[q].c);
               CK(cudaGetLastError());
               b.cf_jm[q].p = f;
             } else if (!c->comp && !b.cd_jm[q].p) {
               double* f = nullptr;
-              if ((rc = dalloc(c, &f, (size_t)b.N))) return rc;
-              k_fill_const<double><<<grid1d(b.N), 256, 0, c->stream>>>(b.N, f, b.cd_jm[q].c);
+              if ((rc = dalloc(c, &f, (size_t)b.NP))) return rc;
+              k_fill_const<double><<<grid1d(b.NP), 256, 0, c->stream>>>(b.NP, f, b.cd_jm[q].c);
               CK(cudaGetLastError());
               b.cd_jm[q].p = f;
             }
@@ -477,8 +522,16 @@ int lee_prepare(lee_ctx* c) {
       return rc;
     CK(cudaMemcpyAsync(o.d_rb, o.rb.data(), n * sizeof(int), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(o.d_db, o.db.data(), n * sizeof(int), cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(o.d_rl, o.rl.data(), n * sizeof(long long), cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(o.d_dl, o.dl.data(), n * sizeof(long long), cudaMemcpyHostToDevice, s));
+    // (points as the state fields hold them)
+    std::vector<long long> trl = o.rl, tdl = o.dl;
+    for (size_t r = 0; r < n; ++r) {
+      const BlockData &rk = c->blk[(size_t)o.rb[r]], &dk = c->blk[(size_t)o.db[r]];
+      trl[r] = row_pos(trl[r], rk.nx, rk.px);
+      tdl[r] = row_pos(tdl[r], dk.nx, dk.px);
+    }
+    CK(cudaMemcpyAsync(o.d_rl, trl.data(), n * sizeof(long long), cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(o.d_dl, tdl.data(), n * sizeof(long long), cudaMemcpyHostToDevice, s));
+    CK(cudaStreamSynchronize(s));
     CK(cudaMemcpyAsync(o.d_wt, o.wt.data(), n * o.W * sizeof(double), cudaMemcpyHostToDevice, s));
     // one kernel is enough when no stencil reads a receiver: the sums then cannot see a value
     // written in the same update

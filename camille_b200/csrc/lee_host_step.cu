@@ -154,7 +154,7 @@ int step_impl(lee_ctx* c, const std::vector<double>& dts, const T* amp_tab, cons
             op.y[bi][v] = (T*)t[v];
             op.e[bi][v] = e ? (T*)e[v] : nullptr;
           }
-          op.nx[bi] = b.nx;
+          op.px[bi] = b.px;
           op.ny[bi] = b.ny;
         }
         CK(launch_overset<T>(op, c->stream));
@@ -169,7 +169,7 @@ int step_impl(lee_ctx* c, const std::vector<double>& dts, const T* amp_tab, cons
           // rho'/rho_bar of the pre-filter state, read by the next step's first stage: the
           // reference recomputes its auxiliary fields after the boundary update and not after
           // the filter (temporal_discretization.cpp:236-242)
-          CK(launch_rho<T>(b.N, c->V, (T* const*)tgt, (T* const*)err, b.d_mean[4], c->cfg.gamma, (T*)b.rho,
+          CK(launch_rho<T>(b.NP, c->V, (T* const*)tgt, (T* const*)err, b.d_tpbar, c->cfg.gamma, (T*)b.rho,
                            c->stream));
           b.rho_valid = true;
           c->stats.kernel_launches += 1;
@@ -569,8 +569,15 @@ int lee_eval_rhs(lee_ctx* c, int b, double time, double* const rhs[5]) {
     }
     int rc = launch_stage_any<double>(c, bk, p, bk.y);
     if (rc) return rc;
-    for (int v = 0; v < c->V; ++v)
-      CK(cudaMemcpyAsync(rhs[slot_of(c->V, v)], bk.zb[0][v], (size_t)bk.N * 8, cudaMemcpyDeviceToHost, c->stream));
+    for (int v = 0; v < c->V; ++v) {
+      const void* r = bk.zb[0][v];
+      if (bk.px != bk.nx) {
+        launch_to_double<double>(c->stream, bk.N, tmp, (const double*)bk.zb[0][v], nullptr, bk.nx, bk.px);
+        CK(cudaGetLastError());
+        r = tmp;
+      }
+      CK(cudaMemcpyAsync(rhs[slot_of(c->V, v)], r, (size_t)bk.N * 8, cudaMemcpyDeviceToHost, c->stream));
+    }
   } else {
     StageParams<float> p;
     fill_stage_common<float>(c, bk, p);
@@ -585,7 +592,7 @@ int lee_eval_rhs(lee_ctx* c, int b, double time, double* const rhs[5]) {
     int rc = launch_stage_any<float>(c, bk, p, bk.y);
     if (rc) return rc;
     for (int v = 0; v < c->V; ++v) {
-      launch_to_double<float>(c->stream, bk.N, tmp, (const float*)bk.zb[0][v], nullptr);
+      launch_to_double<float>(c->stream, bk.N, tmp, (const float*)bk.zb[0][v], nullptr, bk.nx, bk.px);
       CK(cudaMemcpyAsync(rhs[slot_of(c->V, v)], tmp, (size_t)bk.N * 8, cudaMemcpyDeviceToHost, c->stream));
     }
   }
@@ -603,10 +610,10 @@ int lee_apply_filter(lee_ctx* c) {
     if (b.need_rho && !b.rho_valid) {
       // the auxiliary fields keep describing the state from before the filter
       if (c->comp)
-        CK(launch_rho<float>(b.N, c->V, (float* const*)b.y, (float* const*)b.comp, b.d_mean[4], c->cfg.gamma,
+        CK(launch_rho<float>(b.NP, c->V, (float* const*)b.y, (float* const*)b.comp, b.d_tpbar, c->cfg.gamma,
                              (float*)b.rho, c->stream));
       else
-        CK(launch_rho<double>(b.N, c->V, (double* const*)b.y, nullptr, b.d_mean[4], c->cfg.gamma, (double*)b.rho,
+        CK(launch_rho<double>(b.NP, c->V, (double* const*)b.y, nullptr, b.d_tpbar, c->cfg.gamma, (double*)b.rho,
                               c->stream));
       b.rho_valid = true;
     }

@@ -100,10 +100,17 @@ __host__ __device__ inline void wave_eval(const Wave& w, const double x[3], doub
   *p = pf;
 }
 
+// Position of a block's l-th point in an array whose rows lie px points apart (blocks hold fewer
+// than 2^31 points).
+__host__ __device__ inline long long row_pos(long long l, int nx, int px) {
+  return px == nx ? l : l + (long long)((unsigned)l / (unsigned)nx) * (px - nx);
+}
+
 // Everything one stage kernel launch needs for one block.
 template <typename T>
 struct StageParams {
   int nx, ny, nz, dim, V;
+  int px;                 // row pitch of every per-point array below, in points (>= nx)
   // RK stage
   int stage, last;        // stage index, 1 on the last stage
   T h, b, a;              // step size, b_i and a_{i+1,i} of the Butcher tableau
@@ -146,6 +153,7 @@ struct StageParams {
 template <typename T>
 struct FilterParams {
   int nx, ny, nz, V, dir, first, last;
+  int px;                     // row pitch in points
   const T* in[kMaxVars];
   T* out[kMaxVars];
   // FP64: y0 for the blend on the last pass; compensated: see lee_step.cu
@@ -165,8 +173,9 @@ template <typename T>
 struct BcParams {
   int kind, dir, end, nd, V;
   int lo[3], nb[3];           // the end face of the line's box (nb[dir] = 1)
-  int nx, ny;
-  long long sd;               // index stride along dir
+  int nx, ny;                 // rows of the setup fields (met, minv, jac, iblank, xyz)
+  int px;                     // row pitch of the state fields in points
+  long long sd;               // index stride of the state along dir
   int S;                      // closure row width
   double c0[9];               // row 0 of the difference operator's left closure
   T* y[kMaxVars];
@@ -218,7 +227,7 @@ struct OvsParams {
   double* buf;               // n x V, when not fused
   T* y[kMaxOvsBlocks][kMaxVars];
   T* e[kMaxOvsBlocks][kMaxVars];  // compensated pair errors, or null
-  int nx[kMaxOvsBlocks], ny[kMaxOvsBlocks];
+  int px[kMaxOvsBlocks], ny[kMaxOvsBlocks];  // row pitch in points, rows per plane
   int pair;
 };
 
@@ -255,6 +264,7 @@ struct TransOp {
 template <typename T>
 struct AdjStageParams {
   int nx, ny, nz, V;
+  int px;                    // row pitch in points
   int first, has_next;
   T hb_in, hb_next, ha_next;
   const T* kin[kMaxVars];
@@ -275,6 +285,7 @@ struct AdjStageParams {
 template <typename T>
 struct AdjFilterParams {
   int nx, ny, nz, V, dir, last;
+  int px;                    // row pitch in points
   const T* in[kMaxVars];
   T* out[kMaxVars];
   const T* lam[kMaxVars];
@@ -343,6 +354,7 @@ struct AdjGenParams {
 template <typename T>
 struct AdjGenFilterParams {
   int nx, ny, nz, V, dir, last, mask_in;
+  int px;                    // row pitch in points
   const T* in[kMaxVars];
   T* out[kMaxVars];
   const T* lam[kMaxVars];
@@ -405,6 +417,8 @@ cudaError_t launch_adjg_overset(const AdjGenOvs<T>& p, cudaStream_t s);
 template <typename T>
 struct BatchFilterInst {
   int nx, ny;
+  int px;           // row pitch in points
+  int pad_;
   const T* x[4];
   const T* err[4];
   T* y[4];
@@ -459,7 +473,9 @@ cudaError_t setup_scale(int n, double* out, const double* sum, const double* jac
 cudaError_t setup_sigma(int nx, int ny, int nz, const double* const* xyz, const int lo[3], const int hi[3], int dir,
                         int end, int order, double constant, double* sig, cudaStream_t s);
 cudaError_t setup_minmax(int n, const double* f, double* d_out2, cudaStream_t s);
-cudaError_t setup_state_minmax(long long n, const void* y, const void* e, bool fp32, double* d_out2, cudaStream_t s);
+// over the nx points of each of `rows` rows px points apart
+cudaError_t setup_state_minmax(long long rows, int nx, int px, const void* y, const void* e, bool fp32, double* d_out2,
+                               cudaStream_t s);
 cudaError_t setup_cfl(int n, int dim, const double* const* met, const double* jac, const double* const* ubar,
                       const double* pbar, const double* sbar, const int* iblank, double gamma, double dt,
                       double* d_max, cudaStream_t s);

@@ -208,10 +208,12 @@ __global__ void k_minmax(long long n, const double* f, double* out2) {
 // Minimum and maximum of one state field, the value of a point being y (FP64) or fl64(y) + fl64(e)
 // (a compensated FP32 pair): out2[0] collects -min and out2[1] max, both by atomic maximum.
 template <typename T>
-__global__ void k_state_minmax(long long n, const T* y, const T* e, double* out2) {
+__global__ void k_state_minmax(long long rows, int nx, int px, const T* y, const T* e, double* out2) {
   __shared__ double smin[kThreads], smax[kThreads];
   double lo = DBL_MAX, hi = -DBL_MAX;
+  const long long n = rows * px;
   for (long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x; l < n; l += (long long)gridDim.x * blockDim.x) {
+    if (px != nx && l % px >= nx) continue;  // a row's pad
     const double v = e ? (double)y[l] + (double)e[l] : (double)y[l];
     lo = v < lo ? v : lo;
     hi = v > hi ? v : hi;
@@ -356,11 +358,13 @@ cudaError_t setup_minmax(int n, const double* f, double* d_out2, cudaStream_t s)
   return cudaGetLastError();
 }
 
-cudaError_t setup_state_minmax(long long n, const void* y, const void* e, bool fp32, double* d_out2, cudaStream_t s) {
+cudaError_t setup_state_minmax(long long rows, int nx, int px, const void* y, const void* e, bool fp32, double* d_out2,
+                               cudaStream_t s) {
+  const long long n = rows * px;
   if (fp32)
-    k_state_minmax<float><<<grid_for(n), kThreads, 0, s>>>(n, (const float*)y, (const float*)e, d_out2);
+    k_state_minmax<float><<<grid_for(n), kThreads, 0, s>>>(rows, nx, px, (const float*)y, (const float*)e, d_out2);
   else
-    k_state_minmax<double><<<grid_for(n), kThreads, 0, s>>>(n, (const double*)y, (const double*)e, d_out2);
+    k_state_minmax<double><<<grid_for(n), kThreads, 0, s>>>(rows, nx, px, (const double*)y, (const double*)e, d_out2);
   return cudaGetLastError();
 }
 

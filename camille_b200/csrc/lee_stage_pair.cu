@@ -82,7 +82,9 @@ __global__ void __launch_bounds__(128, 3)
   const int k1 = DIM == 3 ? min(s.nz, k0 + P.k_chunk) : 1;
   const int tid = threadIdx.x, tx = tid % LX, ty = tid / LX;
   const int i = i0 + 2 * tx, j = j0 + ty;
-  const bool active = i < s.nx && j < s.ny;  // nx is even: both points of the pair or neither
+  // with an odd nx the last pair's second point is the row's pad (the pitch px is even): it takes
+  // the zero class, so it reads zeros (the copies fill beyond nx) and its pad values stay zero
+  const bool active = i < s.nx && j < s.ny;
   const int plo = DIM == 3 ? max(0, k0 - H) : 0;
   const int phi = DIM == 3 ? min(s.nz - 1, k1 - 1 + H) : 0;
 
@@ -106,7 +108,7 @@ __global__ void __launch_bounds__(128, 3)
   // derivative weights: along xi per point (closure classes), along eta per row
   F2 wx[2 * H + 1], wy[2 * H + 1];
   {
-    const int cx0 = active ? cls_of(i, s.nx, H) : 0, cx1 = active ? cls_of(i + 1, s.nx, H) : 0;
+    const int cx0 = active ? cls_of(i, s.nx, H) : 0, cx1 = !active ? 0 : i + 1 < s.nx ? cls_of(i + 1, s.nx, H) : 1 + 2 * H;
     const int cy = active ? cls_of(j, s.ny, H) : 0;
 #pragma unroll
     for (int o = 0; o <= 2 * H; ++o) {
@@ -120,8 +122,8 @@ __global__ void __launch_bounds__(128, 3)
   for (int x = 0; x < DIM; ++x) nub[x] = f2(-s.ubar[x].c);
   const F2 nrbi = f2(-s.rhobar_inv.c), ngpb = f2(-(s.gamma * s.pbar.c));
   const F2 hh = f2(s.h), bb_ = f2(s.b), aa = f2(s.a);
-  const unsigned nxy = (unsigned)s.nx * (unsigned)s.ny;
-  const unsigned lij = (unsigned)i + (unsigned)s.nx * (unsigned)j;
+  const unsigned nxy = (unsigned)s.px * (unsigned)s.ny;
+  const unsigned lij = (unsigned)i + (unsigned)s.px * (unsigned)j;
   // monopole box test in (i, j), per point of the pair
   const bool src_ij0 = s.has_src && j >= s.src_lo[1] && j <= s.src_hi[1] && i + 1 >= s.src_lo[0] && i <= s.src_hi[0];
 
@@ -339,8 +341,8 @@ cudaError_t go_pair_kind(const FieldMaps& z, const TmaStageParams<float>& p, int
 
 }  // namespace
 
-bool stage_pair_applies(int traits, int nx) {
-  return (traits & kTrTma) && (traits & kTrUniform) && ((traits >> kKindShift) & 7) != kKindRuntime && nx % 2 == 0;
+bool stage_pair_applies(int traits, int px) {
+  return (traits & kTrTma) && (traits & kTrUniform) && ((traits >> kKindShift) & 7) != kKindRuntime && px % 2 == 0;
 }
 
 cudaError_t launch_stage_pair(const FieldMaps& zin, const TmaStageParams<float>& p, int traits, int tiles, int chunks,

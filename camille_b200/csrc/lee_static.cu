@@ -138,6 +138,7 @@ extern "C" int lee_filter_field_static(int num_dim, int filter_scheme, int filte
     FilterParams<double> fp;
     memset(&fp, 0, sizeof fp);
     fp.nx = nxi;
+    fp.px = nxi;
     fp.ny = neta;
     fp.nz = nzeta;
     fp.V = 1;

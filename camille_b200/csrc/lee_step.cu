@@ -56,11 +56,11 @@ __global__ void __launch_bounds__(256) k_stage(StageParams<T> p) {
   const int k = blockIdx.z;
   if (i >= p.nx || j >= p.ny) return;
   constexpr int V = DIM + 2;
-  const long long nxy = (long long)p.nx * p.ny;
-  const long long l = i + (long long)p.nx * j + nxy * k;
+  const long long nxy = (long long)p.px * p.ny;
+  const long long l = i + (long long)p.px * j + nxy * k;
   const int pos[3] = {i, j, k};
   const int nn[3] = {p.nx, p.ny, p.nz};
-  const long long sd[3] = {1, p.nx, nxy};
+  const long long sd[3] = {1, p.px, nxy};
   PointIn<T, DIM> in;
   gather<T, DIM, COMP, kTrGeneric>(p, l, in);
   T D[V][DIM], q[V];
@@ -85,11 +85,11 @@ __global__ void __launch_bounds__(256) k_filter(FilterParams<T> p) {
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
   if (i >= p.nx || j >= p.ny) return;
-  const long long nxy = (long long)p.nx * p.ny;
-  const long long l = i + (long long)p.nx * j + nxy * k;
+  const long long nxy = (long long)p.px * p.ny;
+  const long long l = i + (long long)p.px * j + nxy * k;
   const int pos = p.dir == 0 ? i : (p.dir == 1 ? j : k);
   const int n = p.dir == 0 ? p.nx : (p.dir == 1 ? p.ny : p.nz);
-  const long long sd = p.dir == 0 ? 1 : (p.dir == 1 ? (long long)p.nx : nxy);
+  const long long sd = p.dir == 0 ? 1 : (p.dir == 1 ? (long long)p.px : nxy);
   const bool hole = p.last && p.iblank && p.iblank[l] == 1;
   // a hole after a hole: the reference writes F = 0 there, so the increment is D = -x, and a
   // later pass of a 3-D block reads the zero (the other codes give D = F - I directly)

@@ -82,8 +82,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2)
     }
   }
   // point offsets fit 32 bits (the host checks the block size)
-  const unsigned nxy = (unsigned)s.nx * (unsigned)s.ny;
-  const unsigned lij = (unsigned)i + (unsigned)s.nx * (unsigned)j;
+  const unsigned nxy = (unsigned)s.px * (unsigned)s.ny;
+  const unsigned lij = (unsigned)i + (unsigned)s.px * (unsigned)j;
   // pointwise inputs (y_n, accumulator, J*metrics, sponge): in FP32 they are software-pipelined
   // one plane ahead, so the loads for plane k+1 are in flight while plane k is computed; in
   // FP64 (twice the registers) they are issued at the top of the plane, before the wait
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(256) k_filter_tma_row(const __grid_constant__ 
   // the zero fill and feed nothing)
   auto code_cls = [&](int d, int ii, int jj, int kp) -> int {
     if (ii >= P.nx || jj < 0 || jj >= P.ny) return 0;
-    return cls_of_code(P.code[d][ii + (long long)P.nx * (jj + (long long)P.ny * kp)], P.nb);
+    return cls_of_code(P.code[d][ii + (long long)P.px * (jj + (long long)P.ny * kp)], P.nb);
   };
   T uq[NQ], dq[HF + 1], xq[HF + 1], eq[INC ? HF + 1 : 1];
 #pragma unroll
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(256) k_filter_tma_row(const __grid_constant__ 
     T u2 = T(0), d12 = T(0), xc = T(0);
     const int kf = DIM == 3 ? p - HF : 0;  // the plane finalized at the end of this iteration
     const bool fin = active && kf >= k0 && kf < k1;
-    const long long lf = i + (long long)P.nx * (j + (long long)P.ny * kf);
+    const long long lf = i + (long long)P.px * (j + (long long)P.ny * kf);
     const T ef = (COMP && !INC && fin) ? P.err[v][lf] : T(0);
     T ein = T(0);  // INC: the rounding error of y_pre at this thread's point of plane p
     if (p >= plo && p <= phi) {
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(256) k_filter_tma(const __grid_constant__ Fiel
 #pragma unroll
     for (int r = 0; r < RY; ++r) {
       u2[r] = d12[r] = xc[r] = T(0);
-      ef[r] = (COMP && active[r] && kin) ? P.err[v][i + (long long)P.nx * (jr[r] + (long long)P.ny * kf)] : T(0);
+      ef[r] = (COMP && active[r] && kin) ? P.err[v][i + (long long)P.px * (jr[r] + (long long)P.ny * kf)] : T(0);
     }
     if (p >= plo && p <= phi) {
       const int rel = p - plo;
@@ -554,7 +554,7 @@ __global__ void __launch_bounds__(256) k_filter_tma(const __grid_constant__ Fiel
         x0 = xc[r];
         dsum = d12[r];
       }
-      const long long l = i + (long long)P.nx * (jr[r] + (long long)P.ny * k);
+      const long long l = i + (long long)P.px * (jr[r] + (long long)P.ny * k);
       if (!COMP) {
         P.out[v][l] = (T(1) - P.blend) * x0 + P.blend * fz;
       } else {

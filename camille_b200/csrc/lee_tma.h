@@ -33,6 +33,7 @@ struct TmaStageParams {
 template <typename T>
 struct TmaFilterParams {
   int nx, ny, nz, V, tiles_x, k_chunk;
+  int px;  // row pitch of the fields in points
   int nb;  // class rows per line end: class 0 interior, 1..nb from the left, nb+1..2nb from the right
   // filter weights by class (interior, left rows, right rows, then the zero class 1 + 2 nb of a
   // hole after a hole), offsets -hf..hf; the compensated form uses F - I
@@ -83,7 +84,7 @@ cudaError_t launch_filter_tma(const FieldMaps& in, const TmaFilterParams<T>& p, 
 cudaError_t launch_filter_tma_inc(const FieldMaps& y, const FieldMaps& inc, const TmaFilterParams<float>& p, int hf,
                                   int dim, int tiles, int chunks, cudaStream_t s);
 // The FP32 fused filter with two neighbouring points per thread along xi (lee_filter_pair.cu):
-// 3-D blocks without holes of even nx, half-widths 2, 4 and 5; the compensated form gives the same
+// 3-D blocks without holes of an even row pitch, half-widths 2, 4 and 5; the compensated form gives the same
 // bits as the one-row scalar filter. Its TMA box (bx x by) and tile (tx x ty), and the launch.
 bool filter_pair_half_width(int hf);
 void filter_pair_box(int hf, int* bx, int* by, int* tx, int* ty);
@@ -108,8 +109,8 @@ cudaError_t launch_adj_tma(const AdjMaps& m, const AdjTmaParams<T>& p, bool jm_f
                            cudaStream_t s);
 
 // The FP32 stage kernel with two points per thread (lee_stage_pair.cu): compensated form,
-// uniform mean flow, TMA blocks of even width, a fixed stage kind.
-bool stage_pair_applies(int traits, int nx);
+// uniform mean flow, TMA blocks of an even row pitch, a fixed stage kind.
+bool stage_pair_applies(int traits, int px);
 cudaError_t launch_stage_pair(const FieldMaps& zin, const TmaStageParams<float>& p, int traits, int tiles, int chunks,
                               cudaStream_t s);
 
