@@ -39,6 +39,7 @@ UNITS = {
     "lee_filter.cu": [],
     "lee_filter_pair.cu": [],
     "lee_stage_pair.cu": [],
+    "lee_plane.cu": [],
     "lee_adjoint_tma.cu": [],
     "lee_adjoint_gen.cu": [],
     "lee_host_adjoint_gen.cu": [],
@@ -61,7 +62,7 @@ def _compile(args: list[str]) -> None:
 
 def build(verbose: bool = False, ptxas_info: bool = False) -> str:
     os.makedirs(OBJ, exist_ok=True)
-    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".h")]
+    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     headers.append(os.path.join(ROOT, "include", "lee_b200.h"))
     newest_header = max(os.path.getmtime(h) for h in headers)
     jobs, objs = [], []

@@ -48,7 +48,7 @@ __device__ __forceinline__ T dop_c(const SmOp<T, HH, SS>& w, const T* f, int pos
   T acc = T(0);
   if (pos >= HH && pos <= n - 1 - HH) {
 #pragma unroll
-    for (int l = -HH; l <= HH; ++l) acc += w.c[l + HH] * f[l * ST];
+    for (int l = -HH; l <= HH; ++l) acc = fma_t(w.c[l + HH], f[l * ST], acc);
     return acc;
   }
   // closure rows: zero weights are skipped, so a row reads only the points within HH of its
@@ -58,14 +58,14 @@ __device__ __forceinline__ T dop_c(const SmOp<T, HH, SS>& w, const T* f, int pos
     const T* a = f - r * ST;
 #pragma unroll
     for (int s = 0; s < SS; ++s)
-      if (w.bl[r][s] != T(0)) acc += w.bl[r][s] * a[s * ST];
+      if (w.bl[r][s] != T(0)) acc = fma_t(w.bl[r][s], a[s * ST], acc);
     return acc;
   }
   const int r = n - 1 - pos;
   const T* a = f + r * ST;
 #pragma unroll
   for (int s = 0; s < SS; ++s)
-    if (w.br[r][s] != T(0)) acc += w.br[r][s] * a[-s * ST];
+    if (w.br[r][s] != T(0)) acc = fma_t(w.br[r][s], a[-s * ST], acc);
   return acc;
 }
 
@@ -77,20 +77,20 @@ __device__ __forceinline__ T dop_ring(const SmOp<T, HH, SS>& w, const T* ring, c
   T acc = T(0);
   if (j >= HH && j <= n - 1 - HH) {
 #pragma unroll
-    for (int l = -HH; l <= HH; ++l) acc += w.c[l + HH] * ring[so[l + HH] + col];
+    for (int l = -HH; l <= HH; ++l) acc = fma_t(w.c[l + HH], ring[so[l + HH] + col], acc);
     return acc;
   }
   if (j < HH) {
     const int r = j;
 #pragma unroll
     for (int s = 0; s < SS; ++s)
-      if (w.bl[r][s] != T(0)) acc += w.bl[r][s] * ring[((j - r + s + NSL) % NSL) * rs + col];
+      if (w.bl[r][s] != T(0)) acc = fma_t(w.bl[r][s], ring[((j - r + s + NSL) % NSL) * rs + col], acc);
     return acc;
   }
   const int r = n - 1 - j;
 #pragma unroll
   for (int s = 0; s < SS; ++s)
-    if (w.br[r][s] != T(0)) acc += w.br[r][s] * ring[((j + r - s + 2 * NSL) % NSL) * rs + col];
+    if (w.br[r][s] != T(0)) acc = fma_t(w.br[r][s], ring[((j + r - s + 2 * NSL) % NSL) * rs + col], acc);
   return acc;
 }
 
@@ -292,27 +292,27 @@ __device__ __forceinline__ void batch_filter_run(const BatchFilterInst<T>* __res
           T fy = T(0);
           if (j >= H && j <= ny - 1 - H) {
 #pragma unroll
-            for (int q = -H; q <= H; ++q) fy += w.c[q + H] * fq[v][q + H];
+            for (int q = -H; q <= H; ++q) fy = fma_t(w.c[q + H], fq[v][q + H], fy);
           } else if (j < H) {  // left closure row j reads rows s = 0 .. S-1, i.e. q = s - j
 #pragma unroll
             for (int q = -H; q <= H; ++q) {
               const int sidx = j + q;
-              if (sidx >= 0 && sidx < S && w.bl[j][sidx] != T(0)) fy += w.bl[j][sidx] * fq[v][q + H];
+              if (sidx >= 0 && sidx < S && w.bl[j][sidx] != T(0)) fy = fma_t(w.bl[j][sidx], fq[v][q + H], fy);
             }
           } else {  // right closure row rr reads rows ny-1-s, s = 0 .. S-1, i.e. q = rr - s (s ascending)
             const int rr = ny - 1 - j;
 #pragma unroll
             for (int q = H; q >= -H; --q) {
               const int sidx = rr - q;
-              if (sidx >= 0 && sidx < S && w.br[rr][sidx] != T(0)) fy += w.br[rr][sidx] * fq[v][q + H];
+              if (sidx >= 0 && sidx < S && w.br[rr][sidx] != T(0)) fy = fma_t(w.br[rr][sidx], fq[v][q + H], fy);
             }
           }
           const T xc = xrow[v * W];
           if (!COMP) {
-            P.y[vb + v][l] = (T(1) - blend) * xc + blend * fy;
+            P.y[vb + v][l] = fma_t(blend, fy, (T(1) - blend) * xc);
           } else {
             const T dsum = dq[v][0] + fy;
-            const T tt = blend * dsum + err_nxt[v];
+            const T tt = fma_t(blend, dsum, err_nxt[v]);
             const T s2 = xc + tt;
             const T bb = s2 - xc;
             const T e = (xc - (s2 - bb)) + (tt - bb);

@@ -17,6 +17,7 @@
 #include <memory>
 
 #include "lee_internal.h"
+#include "lee_plane.h"
 #include "lee_tma.h"
 
 using namespace lee;
@@ -94,6 +95,8 @@ struct BlockData {
   // TMA-staged kernels (blocks without holes, 4th-order difference)
   bool tma = false, tma_filter = false;
   bool filter_vec = false;           // the vectorised fused filter (lee_filter.cu) applies
+  bool plane_stage = false;          // 2-D: the direct stage kernel (lee_plane.cu)
+  bool plane_filter = false;         // 2-D: the direct filter kernel
   int filter_px = 0;                 // the fused filter's kernel: 0 scalar, else the vector group width
   int stage_px = 1;                  // points per thread of the TMA stage kernel (2: lee_stage_pair.cu)
   bool stage_pair = false;           // the two-point stage kernel applies
@@ -230,12 +233,19 @@ struct lee_ctx {
     void* d_prm_graph = nullptr;   // StageParams [stage][block], monopole amplitudes from the graph table
     void* d_prm_direct = nullptr;  // the same with the amplitudes of the step being launched
     void* d_finst = nullptr;       // BatchFilterInst [block]
+    std::vector<void*> roles;      // the buffer roles d_finst and d_maps were built for
     std::vector<double> graph_dts;  // time steps d_prm_graph was built for
     // lee_set_batch_persistent: -1 the per-phase launches, else the shape of the one persistent
     // launch per step, its work list and its grid barrier (two words)
     int pshape = -1;
     int4* d_ptiles = nullptr;
     int npt = 0;
+    // the direct kernels of 2-D blocks (lee_plane.cu), until lee_set_batch_shapes asks for strips
+    bool plane = false;
+    bool jm_fields = false;        // some block's J*metrics vary
+    int4 *d_pstiles = nullptr, *d_pftiles = nullptr;
+    CUtensorMap* d_maps = nullptr;  // plane_batch_maps
+    int npst = 0, npft = 0;
     unsigned* d_gbar = nullptr;
   } batch;
   // discrete adjoint (single block, uniform mean, no BC lines, holes or overset)
@@ -353,6 +363,9 @@ int filter_box(const lee_ctx* c, int h, int form, int* bx, int* by);
 int filter_tiles(const BlockData& b);
 int filter_tiles_form(const BlockData& b, int ry);  // the scalar fused filter's tiles in form ry (1 or 2)
 void set_filter_tiles(const lee_ctx* c, BlockData& b);
+int plane_filter_rows(const BlockData& b, int V);
+template <typename T>
+void plane_filter_common(const lee_ctx* c, PlaneFilter<T>& p);
 template <typename T>
 int launch_stage_any(lee_ctx* c, BlockData& b, const StageParams<T>& p, void* const* zin, int chunk_override = 0);
 template <typename T>
@@ -388,6 +401,8 @@ template <typename T>
 int batch_launch_filter(lee_ctx* c, const void* inst, const int4* tiles, int nt, int shape, int grid);
 template <typename T>
 int batch_setup(lee_ctx* c);
+template <typename T>
+int batch_refresh(lee_ctx* c);
 template <typename T>
 int batch_step(lee_ctx* c, const std::vector<double>& dts, bool graph);
 template <typename T>

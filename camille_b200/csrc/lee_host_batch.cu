@@ -130,6 +130,51 @@ int batch_launch_filter(lee_ctx* c, const void* inst, const int4* tiles, int nt,
   return LEE_OK;
 }
 
+// The direct kernels' work lists: tiles (block, x0, y0, 0) of kPlaneCols x ty points.
+std::vector<int4> plane_tiles(const lee_ctx* c, int ty) {
+  std::vector<int4> t;
+  for (size_t b = 0; b < c->blk.size(); ++b)
+    for (int y0 = 0; y0 < c->blk[b].ny; y0 += ty)
+      for (int x0 = 0; x0 < c->blk[b].nx; x0 += kPlaneCols) t.push_back(make_int4((int)b, x0, y0, 0));
+  return t;
+}
+
+// The tensor maps of the direct filter's input, four fields of every block.
+template <typename T>
+int plane_batch_maps(lee_ctx* c) {
+  int bx, by;
+  plane_filter_box(&bx, &by);
+  std::vector<CUtensorMap> m(c->blk.size() * 4);
+  const int ns = tableau(c->cfg.rk_scheme).ns;
+  for (size_t q = 0; q < c->blk.size(); ++q) {
+    BlockData& b = c->blk[q];
+    int rc = encode_maps(c, b, c->comp ? b.zb[(ns - 1) % 2] : b.acc, 4, bx, by, &m[q * 4]);
+    if (rc) return rc;
+  }
+  CK(cudaMemcpy(c->batch.d_maps, m.data(), m.size() * sizeof(m[0]), cudaMemcpyHostToDevice));
+  return LEE_OK;
+}
+
+template <typename T>
+int plane_batch_stage(lee_ctx* c, const StageParams<T>* prm, int s, int ns) {
+  auto& bt = c->batch;
+  PlaneWeights<T> w;
+  for (int a = 0; a < 6; ++a)
+    for (int o = 0; o < 5; ++o) w.w[a][o] = (T)c->wst[a][o];
+  const int kind = s == 0 ? kKindFirst : (s == ns - 1 ? kKindLast : kKindMid);
+  CK(launch_plane_stage_batch<T>(prm, bt.d_pstiles, bt.npst, w, kind, bt.jm_fields, c->stream));
+  return LEE_OK;
+}
+
+template <typename T>
+int plane_batch_filter(lee_ctx* c) {
+  auto& bt = c->batch;
+  PlaneFilter<T> p;
+  plane_filter_common<T>(c, p);
+  CK(launch_plane_filter_batch<T>((const BatchFilterInst<T>*)bt.d_finst, bt.d_maps, bt.d_pftiles, bt.npft, p, c->d_err, c->wait_ns, c->stream));
+  return LEE_OK;
+}
+
 // Setup of the batched path at lee_prepare: operand arrays, sponge fields, and the tile shapes
 // of the stage and filter launches picked by timing every candidate (right-hand-side-only
 // stage launches and filter launches into scratch buffers, so the state is left alone).
@@ -145,7 +190,6 @@ int batch_setup(lee_ctx* c) {
   if ((rc = dev_alloc(c, &bt.d_prm_graph, pbytes)) || (rc = dev_alloc(c, &bt.d_prm_direct, pbytes))) return rc;
   std::vector<BatchFilterInst<T>> fi = batch_filter_inst<T>(c, false);
   if ((rc = dev_alloc(c, &bt.d_finst, fi.size() * sizeof(fi[0])))) return rc;
-  CK(cudaMemcpyAsync(bt.d_finst, fi.data(), fi.size() * sizeof(fi[0]), cudaMemcpyHostToDevice, c->stream));
   // scratch operands for the timing runs
   const std::vector<double> dts((size_t)nbk, 1e-3);
   std::vector<StageParams<T>> pr = batch_params<T>(c, dts, false, 1);
@@ -209,8 +253,48 @@ int batch_setup(lee_ctx* c) {
   CK(cudaMemcpy(bt.d_ftiles, tiles_f.data(), tiles_f.size() * sizeof(int4), cudaMemcpyHostToDevice));
   bt.nst = (int)tiles_s.size();
   bt.nft = (int)tiles_f.size();
+  // the direct kernels serve every batch whose rows are 16-byte multiples (the row pitch's doing);
+  // the strips above run when lee_set_batch_shapes or lee_set_batch_persistent asks for them
+  bt.plane = true;
+  bt.jm_fields = false;
+  for (auto& b : c->blk) {
+    bt.plane = bt.plane && b.tma && b.tma_filter && b.NP < (1ll << 31);
+    for (int q = 0; q < 9; ++q) bt.jm_fields |= (c->comp ? (const void*)b.cf_jm[q].p : (const void*)b.cd_jm[q].p) != nullptr;
+  }
+  if (bt.plane) {
+    const std::vector<int4> ps = plane_tiles(c, kPlaneBatchTall), pf = plane_tiles(c, kPlaneWarps * kPlaneBatchRows);
+    if ((rc = dalloc(c, &bt.d_pstiles, ps.size())) || (rc = dalloc(c, &bt.d_pftiles, pf.size()))) return rc;
+    CK(cudaMemcpy(bt.d_pstiles, ps.data(), ps.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(bt.d_pftiles, pf.data(), pf.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    if ((rc = dalloc(c, &bt.d_maps, c->blk.size() * 4))) return rc;
+    bt.npst = (int)ps.size();
+    bt.npft = (int)pf.size();
+  }
   // the timing runs wrote right-hand sides and filtered values into scratch buffers only
   bt.active = true;
+  return batch_refresh<T>(c);
+}
+
+// The filter's operands follow the blocks' buffer roles (lee_apply_filter swaps them).
+template <typename T>
+int batch_refresh(lee_ctx* c) {
+  auto& bt = c->batch;
+  std::vector<void*> roles;
+  for (auto& b : c->blk)
+    for (int v = 0; v < c->V; ++v) {
+      roles.push_back(b.y[v]);
+      roles.push_back(b.acc[v]);
+      roles.push_back(b.zb[0][v]);
+      roles.push_back(b.zb[1][v]);
+      roles.push_back(b.comp[v]);
+    }
+  if (roles == bt.roles) return LEE_OK;
+  std::vector<BatchFilterInst<T>> fi = batch_filter_inst<T>(c, false);
+  CK(cudaStreamSynchronize(c->stream));  // steps under way read the old operands
+  CK(cudaMemcpy(bt.d_finst, fi.data(), fi.size() * sizeof(fi[0]), cudaMemcpyHostToDevice));
+  if (bt.plane)
+    if (int rc = plane_batch_maps<T>(c)) return rc;
+  bt.roles.swap(roles);
   return LEE_OK;
 }
 
@@ -241,8 +325,9 @@ int batch_step(lee_ctx* c, const std::vector<double>& dts, bool graph) {
   }
   for (int s = 0; s < tb.ns; ++s) {
     int e0 = mark(c);
-    int rc = batch_launch_stage<T>(c, (const StageParams<T>*)prm + (size_t)s * nbk, bt.d_stiles, bt.nst, bt.sshape,
-                                   bt.sgrid);
+    const StageParams<T>* sp = (const StageParams<T>*)prm + (size_t)s * nbk;
+    int rc = bt.plane ? plane_batch_stage<T>(c, sp, s, tb.ns)
+                      : batch_launch_stage<T>(c, sp, bt.d_stiles, bt.nst, bt.sshape, bt.sgrid);
     if (rc) return rc;
     int e1 = mark(c);
     span(c, 0, e0, e1);
@@ -250,7 +335,8 @@ int batch_step(lee_ctx* c, const std::vector<double>& dts, bool graph) {
     c->stats.kernel_launches += 1;
   }
   int e0 = mark(c);
-  int rc = batch_launch_filter<T>(c, bt.d_finst, bt.d_ftiles, bt.nft, bt.fshape, bt.fgrid);
+  int rc = bt.plane ? plane_batch_filter<T>(c)
+                    : batch_launch_filter<T>(c, bt.d_finst, bt.d_ftiles, bt.nft, bt.fshape, bt.fgrid);
   if (rc) return rc;
   int e1 = mark(c);
   span(c, 1, e0, e1);
@@ -266,6 +352,8 @@ template std::vector<BatchFilterInst<float>> batch_filter_inst<float>(lee_ctx* c
 template std::vector<BatchFilterInst<double>> batch_filter_inst<double>(lee_ctx* c, bool scratch);
 template int batch_setup<float>(lee_ctx* c);
 template int batch_setup<double>(lee_ctx* c);
+template int batch_refresh<float>(lee_ctx* c);
+template int batch_refresh<double>(lee_ctx* c);
 template int batch_step<float>(lee_ctx* c, const std::vector<double>& dts, bool graph);
 template int batch_step<double>(lee_ctx* c, const std::vector<double>& dts, bool graph);
 
@@ -291,6 +379,7 @@ int lee_set_batch_shapes(lee_ctx* c, int stage_shape, int filter_shape) {
   bt.nft = (int)tf.size();
   bt.sshape = stage_shape;
   bt.fshape = filter_shape;
+  bt.plane = false;  // the strips were asked for
   const int occs = c->comp ? batch_stage_occupancy<float>(stage_shape, 1) : batch_stage_occupancy<double>(stage_shape, 0);
   const int occf = c->comp ? batch_filter_occupancy<float>(filter_shape, 1)
                            : batch_filter_occupancy<double>(filter_shape, 0);

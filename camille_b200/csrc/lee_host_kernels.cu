@@ -156,6 +156,20 @@ int launch_stage_any(lee_ctx* c, BlockData& b, const StageParams<T>& p, void* co
     CK(launch_stage<T>(p, c->comp ? 1 : 0, c->stream));
     return LEE_OK;
   }
+  // the stage's kind selects a specialised kernel; a first stage that is also the last (no
+  // such tableau here) reads p.stage and p.last at run time
+  const int kind = p.stage < 0 ? kKindRhs
+                   : p.stage == 0 ? (p.last ? kKindRuntime : kKindFirst)
+                                  : (p.last ? (p.increment ? kKindLastIncrement : kKindLast) : kKindMid);
+  const int tr = b.traits | (kind << kKindShift);
+  if (b.plane_stage && kind != kKindRuntime && kind != kKindLastIncrement) {
+    PlaneStage<T> pp;
+    pp.s = p;
+    for (int a = 0; a < 6; ++a)
+      for (int o = 0; o < 5; ++o) pp.w[a][o] = (T)c->wst[a][o];
+    CK(launch_plane_stage<T>(pp, tr, c->stream));
+    return LEE_OK;
+  }
   TmaStageParams<T> tp;
   memset(&tp, 0, sizeof tp);
   tp.s = p;
@@ -169,12 +183,6 @@ int launch_stage_any(lee_ctx* c, BlockData& b, const StageParams<T>& p, void* co
   int rc = field_maps(c, b, zin, Box<T, kFdHalf>::BX, Box<T, kFdHalf>::BY, &fm);
   if (rc) return rc;
   const int chunks = c->cfg.num_dim == 3 ? (b.nz + tp.k_chunk - 1) / tp.k_chunk : 1;
-  // the stage's kind selects a specialised kernel; a first stage that is also the last (no
-  // such tableau here) reads p.stage and p.last at run time
-  const int kind = p.stage < 0 ? kKindRhs
-                   : p.stage == 0 ? (p.last ? kKindRuntime : kKindFirst)
-                                  : (p.last ? (p.increment ? kKindLastIncrement : kKindLast) : kKindMid);
-  const int tr = b.traits | (kind << kKindShift);
   if constexpr (sizeof(T) == 4) {
     if (b.stage_px == 2 && stage_pair_applies(tr, b.px)) {
       CK(launch_stage_pair(fm, tp, tr, b.tiles_x * b.tiles_y, chunks, c->stream));
@@ -185,10 +193,50 @@ int launch_stage_any(lee_ctx* c, BlockData& b, const StageParams<T>& p, void* co
   return LEE_OK;
 }
 
+// Rows a warp of the direct 2-D filter finishes: two filter 1.5 rows along xi per row finished
+// instead of 2, one gives twice the CTAs. Per launch at 64 x 48 .. 640 x 640 FP32 2.4 .. 8.8 us
+// against 2.4 .. 13.0 (the TMA forms), FP64 2.5 .. 13.0 against 2.6 .. 15.9.
+int plane_filter_rows(const BlockData& b, int V) {
+  const long long ctas = (long long)((b.nx + kPlaneCols - 1) / kPlaneCols) * ((b.ny + 2 * kPlaneWarps - 1) / (2 * kPlaneWarps)) * V;
+  return ctas >= 148 * 2 ? 2 : 1;
+}
+
+template <typename T>
+void plane_filter_common(const lee_ctx* c, PlaneFilter<T>& p) {
+  memset(&p, 0, sizeof p);
+  p.nb = c->hf;
+  for (int a = 0; a < 12; ++a)
+    for (int o = 0; o < 11; ++o) p.w[a][o] = (T)c->wfl[a][o];
+  p.blend = (T)c->cfg.filter_blend;
+}
+
 // Fused filter (all directions, one read and one write of the state): in -> out.
 template <typename T>
 int launch_filter_fused(lee_ctx* c, BlockData& b, void* const* in, void* const* err, void* const* out,
                         void* const* comp_out, int chunk_override, void* const* inc) {
+  if (b.plane_filter && !inc && !chunk_override) {
+    PlaneFilter<T> pf;
+    plane_filter_common<T>(c, pf);
+    pf.nx = b.nx;
+    pf.ny = b.ny;
+    pf.px = b.px;
+    pf.rows = plane_filter_rows(b, c->V);
+    if (b.has_holes) {
+      pf.code[0] = b.d_tcode_flt[0];
+      pf.code[1] = b.d_tcode_flt[1];
+      pf.iblank = b.d_tiblank;
+    }
+    for (int v = 0; v < c->V; ++v)
+      pf.f[v] = PlaneFilterField<T>{(const T*)in[v], err ? (const T*)err[v] : nullptr, (T*)out[v],
+                                    comp_out ? (T*)comp_out[v] : nullptr};
+    int e0 = mark(c);
+    CK(launch_plane_filter<T>(pf, c->hf, c->V, c->stream));
+    int e1 = mark(c);
+    span(c, 1, e0, e1);
+    c->stats.filter_launches += 1;
+    c->stats.kernel_launches += 1;
+    return LEE_OK;
+  }
   TmaFilterParams<T> fp;
   memset(&fp, 0, sizeof fp);
   fp.nx = b.nx; fp.ny = b.ny; fp.nz = b.nz;
@@ -312,6 +360,8 @@ int autotune(lee_ctx* c, BlockData& b) {
           if (b.filter_form == 0 && (b.filter_px > 0 || b.has_holes || (c->comp && c->increment_step)) && form > 1)
             continue;
           if (form == 3 && !b.filter_pair_ok) continue;
+          // (where the two-point form applies it is the fastest: 0.43 against 0.61 ms at 256^3)
+          if (b.filter_form == 0 && b.filter_pair_ok && form != 3 && !(c->comp && c->increment_step)) continue;
           b.filter_ry = form == 2 ? 2 : 1;
           b.filter_pair = form == 3;
           set_filter_tiles(c, b);
@@ -339,7 +389,7 @@ int autotune(lee_ctx* c, BlockData& b) {
               }
               rc = launch_stage_any<T>(c, b, p, b.zb[0], d3 ? ch : 0);
             } else {
-              const int chunk = d3 ? ch : 0;
+              const int chunk = ch;  // (2-D: 1, the TMA forms)
               rc = c->comp ? launch_filter_fused<T>(c, b, b.zb[1], b.acc, b.zb[0], b.comp, chunk)
                            : launch_filter_fused<T>(c, b, b.acc, nullptr, b.zb[0], nullptr, chunk);
             }
@@ -500,6 +550,8 @@ template int run_filter<float>(lee_ctx* c, BlockData& b, void** in, void** err, 
                void*** result);
 template int run_filter<double>(lee_ctx* c, BlockData& b, void** in, void** err, void** comp_out, void** f0, void** f1,
                void*** result);
+template void plane_filter_common<float>(const lee_ctx*, PlaneFilter<float>&);
+template void plane_filter_common<double>(const lee_ctx*, PlaneFilter<double>&);
 template int launch_stage_any<float>(lee_ctx* c, BlockData& b, const StageParams<float>& p, void* const* zin, int chunk_override);
 template int launch_stage_any<double>(lee_ctx* c, BlockData& b, const StageParams<double>& p, void* const* zin, int chunk_override);
 template int launch_filter_fused<float>(lee_ctx* c, BlockData& b, void* const* in, void* const* err, void* const* out,

@@ -365,6 +365,8 @@ int capture_steps(lee_ctx* c, const std::vector<double>& dts) {
 template <typename T>
 int advance_impl(lee_ctx* c, int nsteps, const std::vector<double>& dts) {
   auto& g = c->graph;
+  if (c->batch.active)
+    if (int rc = batch_refresh<T>(c)) return rc;
   int done = 0;
   auto direct = [&](int n) -> int {
     for (int k = 0; k < n; ++k) {

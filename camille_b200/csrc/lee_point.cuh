@@ -10,6 +10,11 @@
 
 namespace lee {
 
+// a b + c with one rounding: the kernels that share this file's terms give the same bits whatever
+// the compiler would have contracted around them
+__device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
+
 template <typename T, typename I>
 __device__ __forceinline__ T cval(const Coef<T>& c, I l) {
   return c.p ? __ldg(c.p + l) : c.c;
@@ -76,12 +81,11 @@ __device__ __forceinline__ void rk_update(const StageParams<T>& p, I l, const T 
                                           const PointIn<T, DIM>& in, const T (&r)[DIM + 2]);
 
 // D[v][d]: computational-space derivative of field v along direction d; q[v]: the
-// stage input at the point; in: the gathered inputs. Writes the next stage input and
-// the accumulator.
-template <typename T, int DIM, bool COMP, int TR, typename I>
-__device__ __forceinline__ void rhs_update(const StageParams<T>& p, I l, int i, int j, int k,
-                                           const T (&D)[DIM + 2][DIM], const T (&q)[DIM + 2],
-                                           const PointIn<T, DIM>& in) {
+// stage input at the point; in: the gathered inputs. r receives the right-hand side.
+template <typename T, int DIM, int TR, typename I>
+__device__ __forceinline__ void rhs_point(const StageParams<T>& p, I l, int i, int j, int k,
+                                          const T (&D)[DIM + 2][DIM], const T (&q)[DIM + 2],
+                                          const PointIn<T, DIM>& in, T (&r)[DIM + 2]) {
   constexpr int V = DIM + 2;
   constexpr int P = DIM + 1;
   // physical gradients g[v][x] = sum_d JM[d][x] D_d f_v (take_derivative_xyz, :1802-1826)
@@ -92,7 +96,7 @@ __device__ __forceinline__ void rhs_update(const StageParams<T>& p, I l, int i, 
     for (int v = 0; v < V; ++v) {
       T s = T(0);
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) s += in.jm[d][x] * D[v][d];
+      for (int d = 0; d < DIM; ++d) s = fma_t(in.jm[d][x], D[v][d], s);
       g[v][x] = s;
     }
   }
@@ -100,28 +104,27 @@ __device__ __forceinline__ void rhs_update(const StageParams<T>& p, I l, int i, 
   T ub[DIM];
 #pragma unroll
   for (int x = 0; x < DIM; ++x) ub[x] = UNI ? p.ubar[x].c : cval(p.ubar[x], l);
-  T r[V];
   if (UNI) {
     // uniform mean flow: every mean-gradient term vanishes
     T rs = T(0);
 #pragma unroll
-    for (int x = 0; x < DIM; ++x) rs -= ub[x] * g[0][x];
+    for (int x = 0; x < DIM; ++x) rs = fma_t(-ub[x], g[0][x], rs);
     r[0] = rs;
     const T rbi = p.rhobar_inv.c;
 #pragma unroll
     for (int a = 0; a < DIM; ++a) {
       T ru = T(0);
 #pragma unroll
-      for (int x = 0; x < DIM; ++x) ru -= ub[x] * g[1 + a][x];
-      ru -= g[P][a] * rbi;
+      for (int x = 0; x < DIM; ++x) ru = fma_t(-ub[x], g[1 + a][x], ru);
+      ru = fma_t(-g[P][a], rbi, ru);
       r[1 + a] = ru;
     }
     T rp = T(0);
     const T gpb = p.gamma * p.pbar.c;
 #pragma unroll
     for (int x = 0; x < DIM; ++x) {
-      rp -= ub[x] * g[P][x];
-      rp -= gpb * g[1 + x][x];
+      rp = fma_t(-ub[x], g[P][x], rp);
+      rp = fma_t(-gpb, g[1 + x][x], rp);
     }
     r[P] = rp;
   } else {
@@ -141,11 +144,11 @@ __device__ __forceinline__ void rhs_update(const StageParams<T>& p, I l, int i, 
     int b0 = p.src_hi[0] - p.src_lo[0] + 1, b1 = p.src_hi[1] - p.src_lo[1] + 1;
     long long lb = (i - p.src_lo[0]) + (long long)b0 * ((j - p.src_lo[1]) + (long long)b1 * (k - p.src_lo[2]));
     const T amp = p.amp_tab ? p.amp_tab[*p.step_ctr * p.nstages + p.stage] : p.src_amp;
-    r[P] += amp * p.src_g[lb];
+    r[P] = fma_t(amp, p.src_g[lb], r[P]);
   }
   if (TR & kTrSponge) {
 #pragma unroll
-    for (int v = 0; v < V; ++v) r[v] += -in.sg * (q[v] - T(0));
+    for (int v = 0; v < V; ++v) r[v] = fma_t(-in.sg, q[v], r[v]);
   } else {
     for (int z = 0; z < p.nzones; ++z) {
       const Zone<T>& zn = p.zones[z];
@@ -165,6 +168,16 @@ __device__ __forceinline__ void rhs_update(const StageParams<T>& p, I l, int i, 
       for (int v = 0; v < V; ++v) r[v] += -sg * (q[v] - T(0));
     }
   }
+}
+
+// The right-hand side at a point, then the stage update: writes the next stage input and the
+// accumulator.
+template <typename T, int DIM, bool COMP, int TR, typename I>
+__device__ __forceinline__ void rhs_update(const StageParams<T>& p, I l, int i, int j, int k,
+                                           const T (&D)[DIM + 2][DIM], const T (&q)[DIM + 2],
+                                           const PointIn<T, DIM>& in) {
+  T r[DIM + 2];
+  rhs_point<T, DIM, TR>(p, l, i, j, k, D, q, in, r);
   rk_update<T, DIM, COMP, TR>(p, l, q, in, r);
 }
 
@@ -244,17 +257,17 @@ __device__ __forceinline__ void rk_update(const StageParams<T>& p, I l, const T 
       // y_next = y_n + sum b_i h k_i; the next stage input y_n + a h k_i
       const T yv = first ? q[v] : in.yn[v];
       const T prev = first ? q[v] : in.av[v];
-      p.acc[v][l] = prev + p.b * hk;
-      if (!last) p.zout[v][l] = yv + p.a * hk;
+      p.acc[v][l] = fma_t(p.b, hk, prev);
+      if (!last) p.zout[v][l] = fma_t(p.a, hk, yv);
     } else {
       // compensated form: acc carries the increment of y since y_n plus the carried
       // rounding error of y; the last stage forms y_pre = y_n + increment as an exact
       // two-float sum (y_pre in zout, its rounding error in acc)
       const T yv = first ? q[v] : in.yn[v];
-      const T inc = in.av[v] + p.b * hk;
+      const T inc = fma_t(p.b, hk, in.av[v]);
       if (!last) {
         p.acc[v][l] = inc;
-        p.zout[v][l] = yv + p.a * hk;
+        p.zout[v][l] = fma_t(p.a, hk, yv);
       } else if (K::increment) {
         p.acc[v][l] = inc;  // the filter forms y_pre and its rounding error
       } else {

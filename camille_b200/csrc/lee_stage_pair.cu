@@ -13,57 +13,18 @@
 //
 // Every mbarrier wait is bounded (about one second); on expiry the CTA records the failure in the
 // device flag, waits (bounded) for its own copies in flight and returns.
-#include "lee_point.cuh"
+#include "lee_pair.cuh"
 #include "lee_tma.h"
 #include "lee_tma_util.cuh"
 
 namespace lee {
 namespace {
 
-using F2 = float2;
-
-__device__ __forceinline__ F2 f2(float x) { return make_float2(x, x); }
-__device__ __forceinline__ F2 add(F2 a, F2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ F2 mul(F2 a, F2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { return __ffma2_rn(a, b, c); }
-// a - b, exactly one rounding
-__device__ __forceinline__ F2 sub(F2 a, F2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
-__device__ __forceinline__ F2 ld2(const float* p) { return *reinterpret_cast<const F2*>(p); }
-__device__ __forceinline__ F2 ldg2(const float* p) { return __ldg(reinterpret_cast<const F2*>(p)); }
-__device__ __forceinline__ void st2(float* p, F2 v) { *reinterpret_cast<F2*>(p) = v; }
-
-// Pointwise inputs of a pair, gathered one plane ahead.
-template <int DIM>
-struct PairIn {
-  F2 jm[DIM][DIM];  // J * metrics[d][x]
-  F2 yn[DIM + 2];   // y_n (stages after the first)
-  F2 av[DIM + 2];   // accumulator, or the carried rounding error (first stage)
-  F2 sg;            // sponge strength
-};
-
-template <int DIM, int TR>
-__device__ __forceinline__ void gather_pair(const StageParams<float>& p, unsigned l, PairIn<DIM>& in) {
-  constexpr int V = DIM + 2;
-  using K = Kind<TR>;
-#pragma unroll
-  for (int d = 0; d < DIM; ++d)
-#pragma unroll
-    for (int x = 0; x < DIM; ++x) in.jm[d][x] = (TR & kTrJmField) ? ldg2(p.jm[d * 3 + x].p + l) : f2(p.jm[d * 3 + x].c);
-  const bool mid = !K::rhs(p) && !K::first(p);
-  const bool need_av = mid || K::first(p);
-#pragma unroll
-  for (int v = 0; v < V; ++v) {
-    in.yn[v] = (mid && !K::increment) ? ld2(p.yn[v] + l) : f2(0.f);
-    in.av[v] = need_av ? (K::first(p) ? ld2(p.comp[v] + l) : ld2(p.acc[v] + l)) : f2(0.f);
-  }
-  in.sg = (TR & kTrSponge) ? ldg2(p.sigma + l) : f2(0.f);
-}
-
 template <int DIM, int TR>
 __global__ void __launch_bounds__(128, 3)
     k_stage_pair(const __grid_constant__ FieldMaps zm, const __grid_constant__ TmaStageParams<float> P) {
   using T = float;
-  constexpr int H = kFdHalf, TX = kTileX, TY = kTileY, V = DIM + 2, PV = DIM + 1;
+  constexpr int H = kFdHalf, TX = kTileX, TY = kTileY, V = DIM + 2;
   constexpr int HX = Box<T, H>::HX, BX = Box<T, H>::BX;
   constexpr int FB = Box<T, H>::FB, FBP = Box<T, H>::FBP;
   constexpr int NS = DIM == 3 ? 2 * H + 1 + StagePrefetch<T>::P : 1;
@@ -71,7 +32,6 @@ __global__ void __launch_bounds__(128, 3)
   constexpr int PLANE = V * FBP;
   constexpr int LX = TX / 2;  // threads per row
   static_assert(HX % 2 == 0 && BX % 2 == 0, "pairs start on 8 bytes");
-  using K = Kind<TR>;
   extern __shared__ __align__(128) unsigned char smem[];
   T* ring = reinterpret_cast<T*>(smem);
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + sizeof(T) * NS * PLANE);
@@ -116,12 +76,7 @@ __global__ void __launch_bounds__(128, 3)
       wy[o] = f2(P.w[cy][o]);
     }
   }
-  // uniform mean flow, negated where the right-hand side subtracts
-  F2 nub[DIM];
-#pragma unroll
-  for (int x = 0; x < DIM; ++x) nub[x] = f2(-s.ubar[x].c);
-  const F2 nrbi = f2(-s.rhobar_inv.c), ngpb = f2(-(s.gamma * s.pbar.c));
-  const F2 hh = f2(s.h), bb_ = f2(s.b), aa = f2(s.a);
+  const PairMean<DIM> M(s);
   const unsigned nxy = (unsigned)s.px * (unsigned)s.ny;
   const unsigned lij = (unsigned)i + (unsigned)s.px * (unsigned)j;
   // monopole box test in (i, j), per point of the pair
@@ -199,96 +154,7 @@ __global__ void __launch_bounds__(128, 3)
           D[v][DIM - 1] = dz;
         }
       }
-      // physical gradients g[v][x] = sum_d JM[d][x] D_d f_v (take_derivative_xyz, :1802-1826)
-      F2 g[V][DIM];
-#pragma unroll
-      for (int x = 0; x < DIM; ++x)
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-          F2 t = mul(cur.jm[0][x], D[v][0]);
-#pragma unroll
-          for (int d = 1; d < DIM; ++d) t = fma2(cur.jm[d][x], D[v][d], t);
-          g[v][x] = t;
-        }
-      // uniform mean flow: r_s = -u.grad s', r_u = -u.grad u' - grad p' / rho, r_p = -u.grad p' - gamma p div u'
-      F2 r[V];
-      {
-        F2 t = mul(nub[0], g[0][0]);
-#pragma unroll
-        for (int x = 1; x < DIM; ++x) t = fma2(nub[x], g[0][x], t);
-        r[0] = t;
-      }
-#pragma unroll
-      for (int a = 0; a < DIM; ++a) {
-        F2 t = mul(nub[0], g[1 + a][0]);
-#pragma unroll
-        for (int x = 1; x < DIM; ++x) t = fma2(nub[x], g[1 + a][x], t);
-        r[1 + a] = fma2(g[PV][a], nrbi, t);
-      }
-      {
-        F2 t = mul(nub[0], g[PV][0]);
-#pragma unroll
-        for (int x = 1; x < DIM; ++x) t = fma2(nub[x], g[PV][x], t);
-#pragma unroll
-        for (int x = 0; x < DIM; ++x) t = fma2(ngpb, g[1 + x][x], t);
-        r[PV] = t;
-      }
-      // monopole: per point of the pair
-      if (src_ij0 && k >= s.src_lo[2] && k <= s.src_hi[2]) {
-        const T amp = s.amp_tab ? s.amp_tab[*s.step_ctr * s.nstages + s.stage] : s.src_amp;
-        const int b0 = s.src_hi[0] - s.src_lo[0] + 1, b1 = s.src_hi[1] - s.src_lo[1] + 1;
-        const long long row = (long long)b0 * ((j - s.src_lo[1]) + (long long)b1 * (k - s.src_lo[2]));
-        if (i >= s.src_lo[0] && i <= s.src_hi[0]) r[PV].x += amp * s.src_g[row + (i - s.src_lo[0])];
-        if (i + 1 >= s.src_lo[0] && i + 1 <= s.src_hi[0]) r[PV].y += amp * s.src_g[row + (i + 1 - s.src_lo[0])];
-      }
-      if (TR & kTrSponge) {
-        const F2 nsg = mul(cur.sg, f2(-1.f));
-#pragma unroll
-        for (int v = 0; v < V; ++v) r[v] = fma2(nsg, q[v], r[v]);
-      } else {
-        for (int zz = 0; zz < s.nzones; ++zz) {
-          const Zone<T>& zn = s.zones[zz];
-          if (j < zn.lo[1] || j > zn.hi[1] || k < zn.lo[2] || k > zn.hi[2]) continue;
-          const int b0 = zn.hi[0] - zn.lo[0] + 1, b1 = zn.hi[1] - zn.lo[1] + 1;
-          const long long row = (long long)b0 * ((j - zn.lo[1]) + (long long)b1 * (k - zn.lo[2]));
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int ii = i + e;
-            if (ii < zn.lo[0] || ii > zn.hi[0]) continue;
-            const T sg = zn.sig[row + (ii - zn.lo[0])];
-#pragma unroll
-            for (int v = 0; v < V; ++v) {
-              if (e == 0) r[v].x += -sg * q[v].x;
-              else r[v].y += -sg * q[v].y;
-            }
-          }
-        }
-      }
-      // the compensated RK stage update (rk_update, lee_point.cuh)
-      if (K::rhs(s)) {
-#pragma unroll
-        for (int v = 0; v < V; ++v) st2(s.zout[v] + lk, r[v]);
-      } else {
-        const bool first = K::first(s), last = K::last(s);
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-          const F2 hk = mul(r[v], hh);
-          const F2 yv = first ? q[v] : cur.yn[v];
-          const F2 inc = fma2(bb_, hk, cur.av[v]);
-          if (!last) {
-            st2(s.acc[v] + lk, inc);
-            st2(s.zout[v] + lk, fma2(aa, hk, yv));
-          } else if (K::increment) {
-            st2(s.acc[v] + lk, inc);  // the filter forms y_pre and its rounding error
-          } else {
-            const F2 sm = add(yv, inc);
-            const F2 bv = sub(sm, yv);
-            const F2 e = add(sub(yv, sub(sm, bv)), sub(inc, bv));
-            st2(s.zout[v] + lk, sm);
-            st2(s.acc[v] + lk, e);
-          }
-        }
-      }
+      pair_update<DIM, TR>(s, M, lk, i, j, k, src_ij0, D, q, cur);
     }
     sk = sk + 1 == NS ? 0 : sk + 1;
     return true;
