@@ -162,19 +162,6 @@ int step_impl(lee_ctx* c, const std::vector<double>& dts, const T* amp_tab, cons
         int rc = scalar_overset<T>(c, s, ns);
         if (rc) return rc;
       }
-      for (auto& b : c->blk) {
-        void** tgt = target(b);
-        void** err = errors(b);
-        if (last && b.need_rho) {
-          // rho'/rho_bar of the pre-filter state, read by the next step's first stage: the
-          // reference recomputes its auxiliary fields after the boundary update and not after
-          // the filter (temporal_discretization.cpp:236-242)
-          CK(launch_rho<T>(b.NP, c->V, (T* const*)tgt, (T* const*)err, b.d_tpbar, c->cfg.gamma, (T*)b.rho,
-                           c->stream));
-          b.rho_valid = true;
-          c->stats.kernel_launches += 1;
-        }
-      }
     }
     if (conc) {
       int rc = fork_sides(c);
@@ -184,6 +171,20 @@ int step_impl(lee_ctx* c, const std::vector<double>& dts, const T* amp_tab, cons
       void** last_out = b.zb[(ns - 1) % 2];
       void** other = b.zb[ns % 2];
       if (conc) c->stream = c->side[(size_t)(&b - &c->blk[0]) % c->side.size()];
+      if (b.need_rho) {
+        // rho'/rho_bar of the pre-filter state, read by the next step's first stage: the
+        // reference recomputes its auxiliary fields after the boundary update and not after
+        // the filter (temporal_discretization.cpp:236-242)
+        void** tgt = c->comp ? last_out : b.acc;
+        const cudaError_t e = launch_rho<T>(b.NP, c->V, (T* const*)tgt, c->comp ? (T* const*)b.acc : nullptr, b.d_tpbar,
+                                            c->cfg.gamma, (T*)b.rho, c->stream);
+        if (e != cudaSuccess) {
+          c->stream = origin;
+          return fail(c, LEE_ERR_CUDA, "launch_rho failed: %s", cudaGetErrorString(e));
+        }
+        b.rho_valid = true;
+        c->stats.kernel_launches += 1;
+      }
       if (increment_step_applies(c, b)) {
         // the last stage left the increment in acc: y_n and the increment in, the filtered state
         // and its rounding error out (into the free stage buffer, which becomes y)
