@@ -200,7 +200,7 @@ __device__ __forceinline__ void batch_stage_run(const StageParams<T>* __restrict
             D[v][1] = dop_ring<T, kFdH, 3, NS>(w, ring, so, V * W, v * W + cl + H, j, ny);
             q[v] = *c0;
           }
-          rhs_update<T, 2, COMP, TR>(P, (long long)j * px + i, i, j, 0, D, q, in_cur[m]);
+          rhs_update<T, 2, COMP, TR>(P, (long long)j * px + i, i, j, 0, D, q, in_cur[m], PointMean<T, 2>{});
         }
         in_cur[m] = in_nxt[m];
       }

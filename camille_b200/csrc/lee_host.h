@@ -83,6 +83,9 @@ struct BlockData {
   Coef<double> cd_jm[9], cd_ub[3], cd_pb, cd_rbi, cd_gs[3], cd_gu[9], cd_gp[3];
   Coef<float> cf_jm[9], cf_ub[3], cf_pb, cf_rbi, cf_gs[3], cf_gu[9], cf_gp[3];
   int need_rho = 0;
+  void* d_mean_const = nullptr;     // constants of StageParams::mean, two of each (working precision)
+  void* d_ipb = nullptr;            // 1 / p_bar where p_bar varies (working precision)
+  int mean_terms = 0;
   int n_coef_fields = 0;
   // state buffers (element size 8 or 4), V fields each
   void* y[kMaxVars] = {};
@@ -99,7 +102,7 @@ struct BlockData {
   bool plane_filter = false;         // 2-D: the direct filter kernel
   int filter_px = 0;                 // the fused filter's kernel: 0 scalar, else the vector group width
   int stage_px = 1;                  // points per thread of the TMA stage kernel (2: lee_stage_pair.cu)
-  bool stage_pair = false;           // the two-point stage kernel applies
+  bool stage_pair = false;           // the two-point stage kernel can be chosen by number
   int vtiles_x = 0, vtiles_y = 0;    // tiles of the vectorised kernel at that width
   int traits = kTrGeneric;          // coefficient-layout traits of the TMA stage kernel
   void* d_sigma_field = nullptr;    // summed sponge strengths per point (working precision)
@@ -350,6 +353,10 @@ bool class_weights(const OpTable& op, int H, double* w, int stride);
 Tableau tableau(int rk);
 int compute_metrics(lee_ctx* c, BlockData& b);
 int build_sigma_field(lee_ctx* c, BlockData& b);
+template <typename T>
+int build_mean(lee_ctx* c, BlockData& b);
+template <typename T>
+void mean_coefs(const BlockData& b, Coef<T> (&k)[20]);
 void set_pitch(const lee_ctx* c, BlockData& b);
 template <typename T>
 int run_filter(lee_ctx* c, BlockData& b, void** in, void** err, void** comp_out, void** f0, void** f1,

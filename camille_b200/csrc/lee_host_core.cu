@@ -308,6 +308,21 @@ int alloc_fields(lee_ctx* c, void** f, long long N) {
 // Map the reference's five slots (s', u', v', w', p') to the V device fields.
 int slot_of(int V, int v) { return v == V - 1 ? 4 : v; }
 
+// The mean-flow coefficients of a block in the order of StageParams::mean (without 1 / p_bar).
+template <typename T>
+void mean_coefs(const BlockData& b, Coef<T> (&k)[20]) {
+  const bool dbl = std::is_same<T, double>::value;
+  auto of = [&](const Coef<double>& d, const Coef<float>& f) { return dbl ? *(const Coef<T>*)&d : *(const Coef<T>*)&f; };
+  for (int x = 0; x < 3; ++x) {
+    k[kMeanUb + x] = of(b.cd_ub[x], b.cf_ub[x]);
+    k[kMeanGs + x] = of(b.cd_gs[x], b.cf_gs[x]);
+    k[kMeanGp + x] = of(b.cd_gp[x], b.cf_gp[x]);
+  }
+  for (int q = 0; q < 9; ++q) k[kMeanGu + q] = of(b.cd_gu[q], b.cf_gu[q]);
+  k[kMeanRbi] = of(b.cd_rbi, b.cf_rbi);
+  k[kMeanPb] = of(b.cd_pb, b.cf_pb);
+}
+
 template <typename T>
 void fill_stage_common(lee_ctx* c, BlockData& b, StageParams<T>& p) {
   memset(&p, 0, sizeof p);
@@ -345,6 +360,15 @@ void fill_stage_common(lee_ctx* c, BlockData& b, StageParams<T>& p) {
   p.iblank = b.has_holes ? b.d_tiblank : nullptr;
   p.fd = c->fd;
   p.sigma = (const T*)b.d_sigma_field;
+  Coef<T> k[20];
+  mean_coefs<T>(b, k);
+  for (int q = 0; q < 20; ++q) {
+    p.mean[q] = k[q].p ? k[q].p : (const T*)b.d_mean_const + 2 * q;
+    p.mean_mask[q] = k[q].p ? -1 : 0;
+  }
+  p.mean[kMeanIpb] = b.d_ipb ? (const T*)b.d_ipb : (const T*)b.d_mean_const + 2 * kMeanIpb;
+  p.mean_mask[kMeanIpb] = b.d_ipb ? -1 : 0;
+  p.mean_terms = b.mean_terms;
 }
 
 // Distributed source: the grid box covered by the lattice, and the trilinear prolongation of
@@ -513,6 +537,8 @@ void set_global_error(const char* msg) { snprintf(g_create_error, sizeof g_creat
 // the host translation units use both precisions
 template int make_coef<float>(lee_ctx* c, BlockData& b, const double* d_field, double scale, Coef<float>* out);
 template int make_coef<double>(lee_ctx* c, BlockData& b, const double* d_field, double scale, Coef<double>* out);
+template void mean_coefs<float>(const BlockData&, Coef<float> (&)[20]);
+template void mean_coefs<double>(const BlockData&, Coef<double> (&)[20]);
 template void fill_stage_common<float>(lee_ctx* c, BlockData& b, StageParams<float>& p);
 template void fill_stage_common<double>(lee_ctx* c, BlockData& b, StageParams<double>& p);
 

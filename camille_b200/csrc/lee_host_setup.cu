@@ -28,6 +28,13 @@ __global__ void k_fill_const(long long n, T* out, T v) {
     out[l] = v;
 }
 
+// 1 / in on rows of nx points at pitch px; zeros in the pads
+template <typename T>
+__global__ void k_reciprocal(long long n, int nx, int px, T* out, const T* in) {
+  for (long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x; l < n; l += (long long)gridDim.x * blockDim.x)
+    out[l] = l % px < nx ? T(1) / in[l] : T(0);
+}
+
 // A setup field at the time loop's row pitch, pads `fill` (the field itself when px = nx).
 template <typename P>
 int at_pitch(lee_ctx* c, const BlockData& b, P* in, P fill, P** out) {
@@ -133,6 +140,33 @@ int compute_metrics(lee_ctx* c, BlockData& b) {
   CK(setup_jacobian(N, dim, d_xx, b.d_invjac, b.d_jac, s));
   CK(setup_inverse_metrics(N, dim, d_mm, d_mi, s));
   CK(cudaStreamSynchronize(s));
+  return LEE_OK;
+}
+
+// StageParams::mean of a block: the constants in device memory, 1 / p_bar, the non-zero gradients.
+template <typename T>
+int build_mean(lee_ctx* c, BlockData& b) {
+  Coef<T> k[20];
+  mean_coefs<T>(b, k);
+  b.mean_terms = 0;
+  for (int q = 0; q < 3; ++q) b.mean_terms |= (k[kMeanGs + q].zero ? 0 : 1) | (k[kMeanGp + q].zero ? 0 : 4);
+  for (int q = 0; q < 9; ++q) b.mean_terms |= k[kMeanGu + q].zero ? 0 : 2;
+  T h[2 * 21];
+  for (int q = 0; q < 20; ++q) h[2 * q] = h[2 * q + 1] = k[q].zero ? T(0) : k[q].c;
+  h[2 * kMeanIpb] = h[2 * kMeanIpb + 1] = T(1) / k[kMeanPb].c;
+  int rc;
+  T* d = nullptr;
+  if ((rc = dalloc(c, &d, 2 * 21))) return rc;
+  CK(cudaMemcpyAsync(d, h, sizeof h, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  b.d_mean_const = d;
+  if (k[kMeanPb].p) {
+    T* r = nullptr;
+    if ((rc = dalloc(c, &r, (size_t)b.NP))) return rc;
+    k_reciprocal<T><<<grid1d(b.NP), 256, 0, c->stream>>>(b.NP, b.nx, b.px, r, k[kMeanPb].p);
+    CK(cudaGetLastError());
+    b.d_ipb = r;
+  }
   return LEE_OK;
 }
 
@@ -404,6 +438,7 @@ int lee_prepare(lee_ctx* c) {
     for (int q = 0; q < 9; ++q) b.need_rho |= c->comp ? !b.cf_gu[q].zero : !b.cd_gu[q].zero;
     if (b.need_rho && (rc = dev_alloc(c, &b.rho, (size_t)b.NP * c->esz))) return rc;
     b.rho_valid = false;
+    if ((rc = c->comp ? build_mean<float>(c, b) : build_mean<double>(c, b))) return rc;
     if ((rc = scalar_setup(c, b))) return rc;
     // state buffers
     if ((rc = alloc_fields(c, b.y, b.NP))) return rc;
@@ -475,7 +510,8 @@ int lee_prepare(lee_ctx* c) {
       for (auto& z : b.bnd) spg |= is_sponge(z.kind);
       b.traits = kTrTma | (jmf ? kTrJmField : 0) | (uni ? kTrUniform : 0) | (spg ? kTrSponge : 0);
       b.stage_pair = c->comp && uni && b.px % 2 == 0 && !b.has_holes;
-      b.stage_px = b.stage_pair ? 2 : 1;
+      // (a choice of the two-point kernel by number stays one of uniform blocks)
+      b.stage_px = c->comp && b.px % 2 == 0 && !b.has_holes ? 2 : 1;
       if (c->stage_kernel > 0) {
         const bool ok = c->stage_kernel == 1 || (c->stage_kernel == 2 && b.stage_pair);
         if (!ok && b.px == b.nx)
@@ -509,8 +545,7 @@ int lee_prepare(lee_ctx* c) {
     // 2-D blocks: the direct kernels (lee_plane.cu), unless a kernel or form was asked for. Per
     // launch at 64 x 48 .. 640 x 640: FP32 stage 2.1 .. 6.0 us against 2.2 .. 7.4 (two-point TMA
     // kernel), FP64 2.7 .. 11.8 against 2.6 .. 12.7; on a 512 x 512 block with holes 7.9 against
-    // 10.2. A non-uniform mean without holes keeps the TMA kernel, whose coefficient loads run one
-    // point per thread (384 x 96: 4.2 against 5.5)
+    // 10.2. A non-uniform mean without holes keeps the TMA kernels (384 x 96 FP32: 3.8 against 5.5)
     b.plane_stage = dim == 2 && b.tma && c->stage_kernel < 0 && ((b.traits & kTrUniform) || b.has_holes);
     b.plane_filter = dim == 2 && b.tma_filter && c->filter_kernel < 0 && c->filter_form == 0 && !c->increment_step &&
                      (c->hf == 2 || c->hf == 4 || c->hf == 5) && c->flt.nb <= kPlaneFilterNb;

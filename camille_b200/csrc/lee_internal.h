@@ -148,7 +148,14 @@ struct StageParams {
   const int8_t* code[3];
   const int* iblank;
   OpTable fd;
+  // the mean-flow coefficients of a non-uniform block again (kMean* below), each read at
+  // mean[k][l & mean_mask[k]]: a field (mask -1), or a constant (mask 0, stored twice so that a
+  // pair of points reads it as one), so that the kernels load them all without a branch
+  const T* mean[21];
+  int mean_mask[21];
+  int mean_terms;  // which gradients are not identically zero: bit 0 s_bar, 1 u_bar, 2 p_bar
 };
+constexpr int kMeanUb = 0, kMeanRbi = 3, kMeanPb = 4, kMeanGs = 5, kMeanGu = 8, kMeanGp = 17, kMeanIpb = 20;
 
 template <typename T>
 struct FilterParams {

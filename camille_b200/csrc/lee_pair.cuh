@@ -1,4 +1,4 @@
-// Two neighbouring points of a uniform-mean block in packed FP32 (sm_100's __ffma2_rn, __fadd2_rn,
+// Two neighbouring points in packed FP32 (sm_100's __ffma2_rn, __fadd2_rn,
 // __fmul2_rn): the pointwise part of the compensated RK stage, shared by the two-point kernels of
 // 3-D and 2-D blocks (lee_stage_pair.cu, lee_plane.cu), so that both give the same bits.
 #pragma once
@@ -47,6 +47,79 @@ __device__ __forceinline__ void gather_pair(const StageParams<float>& p, unsigne
   in.sg = (TR & kTrSponge) ? ldg2(p.sigma + l) : f2(0.f);
 }
 
+// The mean flow at a pair of points of a non-uniform block (PointMean, lee_point.cuh).
+template <int DIM>
+struct PairField {
+  F2 ub[DIM], rbi, pb, gs[DIM], gu[DIM][DIM], gp[DIM], rr;
+};
+
+template <int DIM, int TR>
+__device__ __forceinline__ void gather_mean_pair(const StageParams<float>& p, unsigned l, PairField<DIM>& m) {
+  auto at = [&](int k) { return ldg2(p.mean[k] + (l & (unsigned)p.mean_mask[k])); };
+#pragma unroll
+  for (int x = 0; x < DIM; ++x) m.ub[x] = at(kMeanUb + x);
+  m.rbi = at(kMeanRbi);
+  m.pb = at(kMeanPb);
+#pragma unroll
+  for (int x = 0; x < DIM; ++x) {
+    m.gs[x] = (p.mean_terms & 1) ? at(kMeanGs + x) : f2(0.f);
+    m.gp[x] = (p.mean_terms & 4) ? at(kMeanGp + x) : f2(0.f);
+#pragma unroll
+    for (int a = 0; a < DIM; ++a) m.gu[a][x] = (p.mean_terms & 2) ? at(kMeanGu + a * 3 + x) : f2(0.f);
+  }
+  m.rr = !(p.mean_terms & 2) ? f2(0.f) : (reads_rho_prev<float, TR>(p) ? ld2(p.rho_prev + l) : at(kMeanIpb));
+}
+
+// rhs_mean_terms (lee_point.cuh) of a pair
+template <int DIM, int TR>
+__device__ __forceinline__ void pair_mean_terms(const StageParams<float>& p, const F2 (&g)[DIM + 2][DIM],
+                                                const F2 (&q)[DIM + 2], const PairField<DIM>& m, F2 (&r)[DIM + 2]) {
+  constexpr int P = DIM + 1;
+  const F2 neg = f2(-1.f);
+  F2 nub[DIM], nu[DIM];
+#pragma unroll
+  for (int x = 0; x < DIM; ++x) {
+    nub[x] = mul(m.ub[x], neg);
+    nu[x] = mul(q[1 + x], neg);
+  }
+  F2 rr = f2(0.f);
+  if (p.mean_terms & 2) {
+    rr = m.rr;
+    if (!reads_rho_prev<float, TR>(p)) rr = fma2(mul(q[P], f2(p.inv_gamma)), m.rr, mul(q[0], neg));
+  }
+  {
+    F2 t = mul(nub[0], g[0][0]);
+#pragma unroll
+    for (int x = 0; x < DIM; ++x) {
+      if (x) t = fma2(nub[x], g[0][x], t);
+      if (p.mean_terms & 1) t = fma2(nu[x], m.gs[x], t);
+    }
+    r[0] = t;
+  }
+  const F2 ngpb = mul(m.pb, f2(-p.gamma)), ngq = mul(q[P], f2(-p.gamma));
+#pragma unroll
+  for (int a = 0; a < DIM; ++a) {
+    F2 t = mul(nub[0], g[1 + a][0]);
+#pragma unroll
+    for (int x = 0; x < DIM; ++x) {
+      if (x) t = fma2(nub[x], g[1 + a][x], t);
+      if (p.mean_terms & 2) t = fma2(fma2(rr, nub[x], nu[x]), m.gu[a][x], t);
+    }
+    r[1 + a] = fma2(mul(g[P][a], neg), m.rbi, t);
+  }
+  {
+    F2 t = mul(nub[0], g[P][0]);
+#pragma unroll
+    for (int x = 0; x < DIM; ++x) {
+      if (x) t = fma2(nub[x], g[P][x], t);
+      if (p.mean_terms & 4) t = fma2(nu[x], m.gp[x], t);
+      t = fma2(ngpb, g[1 + x][x], t);
+      if (p.mean_terms & 2) t = fma2(ngq, m.gu[x][x], t);
+    }
+    r[P] = t;
+  }
+}
+
 // A block's uniform mean flow, negated where the right-hand side subtracts, and the stage's factors.
 template <int DIM>
 struct PairMean {
@@ -68,7 +141,8 @@ struct PairMean {
 template <int DIM, int TR, bool STRIP = false>
 __device__ __forceinline__ void pair_update(const StageParams<float>& s, const PairMean<DIM>& M, unsigned l, int i,
                                             int j, int k, bool src_ij0, const F2 (&D)[DIM + 2][DIM],
-                                            const F2 (&q)[DIM + 2], const PairIn<DIM>& in) {
+                                            const F2 (&q)[DIM + 2], const PairIn<DIM>& in,
+                                            const PairField<DIM>& mean) {
   using T = float;
   using K = Kind<TR>;
   constexpr int V = DIM + 2, PV = DIM + 1;
@@ -85,21 +159,21 @@ __device__ __forceinline__ void pair_update(const StageParams<float>& s, const P
     }
   // uniform mean flow: r_s = -u.grad s', r_u = -u.grad u' - grad p' / rho, r_p = -u.grad p' - gamma p div u'
   F2 r[V];
-  {
+  if (!(TR & kTrUniform)) {
+    pair_mean_terms<DIM, TR>(s, g, q, mean, r);
+  } else {
     F2 t = mul(M.nub[0], g[0][0]);
 #pragma unroll
     for (int x = 1; x < DIM; ++x) t = fma2(M.nub[x], g[0][x], t);
     r[0] = t;
-  }
 #pragma unroll
-  for (int a = 0; a < DIM; ++a) {
-    F2 t = mul(M.nub[0], g[1 + a][0]);
+    for (int a = 0; a < DIM; ++a) {
+      t = mul(M.nub[0], g[1 + a][0]);
 #pragma unroll
-    for (int x = 1; x < DIM; ++x) t = fma2(M.nub[x], g[1 + a][x], t);
-    r[1 + a] = fma2(g[PV][a], M.nrbi, t);
-  }
-  {
-    F2 t = mul(M.nub[0], g[PV][0]);
+      for (int x = 1; x < DIM; ++x) t = fma2(M.nub[x], g[1 + a][x], t);
+      r[1 + a] = fma2(g[PV][a], M.nrbi, t);
+    }
+    t = mul(M.nub[0], g[PV][0]);
     if (STRIP) t = fma2(M.ngpb, g[1][0], t);
 #pragma unroll
     for (int x = 1; x < DIM; ++x) {

@@ -228,7 +228,7 @@ __device__ __forceinline__ void stage_point(const StageParams<T>& s, const T (&W
     deriv(2, a2);
     deriv(3, a3);
     const bool src = s.has_src && j >= s.src_lo[1] && j <= s.src_hi[1] && i + 1 >= s.src_lo[0] && i <= s.src_hi[0];
-    pair_update<2, TR, REV>(s, PairMean<2>(s), l, i, j, 0, src, D, q, pin);
+    pair_update<2, TR, REV>(s, PairMean<2>(s), l, i, j, 0, src, D, q, pin, PairField<2>{});
     return;
   }
   struct Field {
@@ -298,6 +298,11 @@ __device__ __forceinline__ void stage_point(const StageParams<T>& s, const T (&W
   if (REV) deriv(1, a1);
   PointIn<T, 2> in[2];
   load_inputs<T, COMP, TR>(s, l, in);
+  PointMean<T, 2> mean[2];
+  if (!(TR & kTrUniform)) {
+    gather_mean<T, 2, TR>(s, l, mean[0]);
+    gather_mean<T, 2, TR>(s, both ? l + 1 : l, mean[1]);
+  }
   if (!REV) {
     deriv(0, a0);
     deriv(1, a1);
@@ -305,8 +310,8 @@ __device__ __forceinline__ void stage_point(const StageParams<T>& s, const T (&W
   deriv(2, a2);
   deriv(3, a3);
   T r[2][V];
-  rhs_point<T, 2, TR>(s, l, i, j, 0, D[0], q[0], in[0], r[0]);
-  rhs_point<T, 2, TR>(s, both ? l + 1 : l, both ? i + 1 : i, j, 0, D[1], q[1], in[1], r[1]);
+#pragma unroll
+  for (int e = 0; e < 2; ++e) rhs_point<T, 2, TR>(s, both ? l + e : l, both ? i + e : i, j, 0, D[e], q[e], in[e], mean[e], r[e]);
   if (K::rhs(s)) {
 #pragma unroll
     for (int v = 0; v < V; ++v) stp(s.zout[v] + l, r[0][v], r[1][v], both);

@@ -73,19 +73,50 @@ __device__ __forceinline__ void gather(const StageParams<T>& p, I l, PointIn<T, 
   in.sg = (TR & kTrSponge) ? __ldg(p.sigma + l) : T(0);
 }
 
+// The mean flow at a point of a non-uniform block.
+template <typename T, int DIM>
+struct PointMean {
+  T ub[DIM], rbi, pb, gs[DIM], gu[DIM][DIM], gp[DIM];
+  T rr;  // rho'/rho_bar of the previous step (stages that read it), else 1 / p_bar
+};
+
+template <typename T, int TR>
+__device__ __forceinline__ bool reads_rho_prev(const StageParams<T>& p) {
+  return (Kind<TR>::first(p) || Kind<TR>::rhs(p)) && p.rho_prev;
+}
+
 template <typename T, int DIM, int TR, typename I>
-__device__ __forceinline__ void rhs_mean_terms(const StageParams<T>& p, I l, const T (&g)[DIM + 2][DIM],
-                                               const T (&q)[DIM + 2], const T (&ub)[DIM], T (&r)[DIM + 2]);
+__device__ __forceinline__ void gather_mean(const StageParams<T>& p, I l, PointMean<T, DIM>& m) {
+  auto at = [&](int k) { return __ldg(p.mean[k] + (l & (I)p.mean_mask[k])); };
+#pragma unroll
+  for (int x = 0; x < DIM; ++x) m.ub[x] = at(kMeanUb + x);
+  m.rbi = at(kMeanRbi);
+  m.pb = at(kMeanPb);
+#pragma unroll
+  for (int x = 0; x < DIM; ++x) {
+    m.gs[x] = (p.mean_terms & 1) ? at(kMeanGs + x) : T(0);
+    m.gp[x] = (p.mean_terms & 4) ? at(kMeanGp + x) : T(0);
+#pragma unroll
+    for (int a = 0; a < DIM; ++a) m.gu[a][x] = (p.mean_terms & 2) ? at(kMeanGu + a * 3 + x) : T(0);
+  }
+  m.rr = !(p.mean_terms & 2) ? T(0) : (reads_rho_prev<T, TR>(p) ? p.rho_prev[l] : at(kMeanIpb));
+}
+
+template <typename T, int DIM, int TR>
+__device__ __forceinline__ void rhs_mean_terms(const StageParams<T>& p, const T (&g)[DIM + 2][DIM],
+                                               const T (&q)[DIM + 2], const PointMean<T, DIM>& m, T (&r)[DIM + 2]);
 template <typename T, int DIM, bool COMP, int TR, typename I>
 __device__ __forceinline__ void rk_update(const StageParams<T>& p, I l, const T (&q)[DIM + 2],
                                           const PointIn<T, DIM>& in, const T (&r)[DIM + 2]);
 
 // D[v][d]: computational-space derivative of field v along direction d; q[v]: the
-// stage input at the point; in: the gathered inputs. r receives the right-hand side.
+// stage input at the point; in: the gathered inputs, mean: the mean flow of a non-uniform block.
+// r receives the right-hand side.
 template <typename T, int DIM, int TR, typename I>
 __device__ __forceinline__ void rhs_point(const StageParams<T>& p, I l, int i, int j, int k,
                                           const T (&D)[DIM + 2][DIM], const T (&q)[DIM + 2],
-                                          const PointIn<T, DIM>& in, T (&r)[DIM + 2]) {
+                                          const PointIn<T, DIM>& in, const PointMean<T, DIM>& mean,
+                                          T (&r)[DIM + 2]) {
   constexpr int V = DIM + 2;
   constexpr int P = DIM + 1;
   // physical gradients g[v][x] = sum_d JM[d][x] D_d f_v (take_derivative_xyz, :1802-1826)
@@ -103,7 +134,7 @@ __device__ __forceinline__ void rhs_point(const StageParams<T>& p, I l, int i, i
   constexpr bool UNI = (TR & kTrUniform) != 0;
   T ub[DIM];
 #pragma unroll
-  for (int x = 0; x < DIM; ++x) ub[x] = UNI ? p.ubar[x].c : cval(p.ubar[x], l);
+  for (int x = 0; x < DIM; ++x) ub[x] = UNI ? p.ubar[x].c : mean.ub[x];
   if (UNI) {
     // uniform mean flow: every mean-gradient term vanishes
     T rs = T(0);
@@ -128,7 +159,7 @@ __device__ __forceinline__ void rhs_point(const StageParams<T>& p, I l, int i, i
     }
     r[P] = rp;
   } else {
-    rhs_mean_terms<T, DIM, TR>(p, l, g, q, ub, r);
+    rhs_mean_terms<T, DIM, TR>(p, g, q, mean, r);
   }
   if constexpr (DIM == 2 && !(TR & kTrTma)) {
     if (p.axisym) {
@@ -175,58 +206,48 @@ __device__ __forceinline__ void rhs_point(const StageParams<T>& p, I l, int i, i
 template <typename T, int DIM, bool COMP, int TR, typename I>
 __device__ __forceinline__ void rhs_update(const StageParams<T>& p, I l, int i, int j, int k,
                                            const T (&D)[DIM + 2][DIM], const T (&q)[DIM + 2],
-                                           const PointIn<T, DIM>& in) {
+                                           const PointIn<T, DIM>& in, const PointMean<T, DIM>& mean) {
   T r[DIM + 2];
-  rhs_point<T, DIM, TR>(p, l, i, j, k, D, q, in, r);
+  rhs_point<T, DIM, TR>(p, l, i, j, k, D, q, in, mean, r);
   rk_update<T, DIM, COMP, TR>(p, l, q, in, r);
 }
 
-// The LEE right-hand side of a non-uniform mean flow: every coefficient is read at the point
-// when it varies, and terms whose mean gradient is identically zero are skipped.
-template <typename T, int DIM, int TR, typename I>
-__device__ __forceinline__ void rhs_mean_terms(const StageParams<T>& p, I l, const T (&g)[DIM + 2][DIM],
-                                               const T (&q)[DIM + 2], const T (&ub)[DIM], T (&r)[DIM + 2]) {
+// The LEE right-hand side of a non-uniform mean flow; gradients that are identically zero are
+// skipped by the field they belong to.
+template <typename T, int DIM, int TR>
+__device__ __forceinline__ void rhs_mean_terms(const StageParams<T>& p, const T (&g)[DIM + 2][DIM],
+                                               const T (&q)[DIM + 2], const PointMean<T, DIM>& m, T (&r)[DIM + 2]) {
   constexpr int P = DIM + 1;
   {
     T rs = T(0);
 #pragma unroll
     for (int x = 0; x < DIM; ++x) {
-      rs -= ub[x] * g[0][x];
-      if (!p.gs[x].zero) rs -= q[1 + x] * cval(p.gs[x], l);
+      rs = fma_t(-m.ub[x], g[0][x], rs);
+      if (p.mean_terms & 1) rs = fma_t(-q[1 + x], m.gs[x], rs);
     }
     r[0] = rs;
   }
   T rr = T(0);
-  if (p.need_rho) {
-    if ((Kind<TR>::first(p) || Kind<TR>::rhs(p)) && p.rho_prev) {
-      rr = p.rho_prev[l];
-    } else {
-      rr = q[P] * p.inv_gamma * (T(1) / cval(p.pbar, l)) - q[0];
-    }
-  }
-  const T rbi = cval(p.rhobar_inv, l);
+  if (p.mean_terms & 2) rr = reads_rho_prev<T, TR>(p) ? m.rr : fma_t(q[P] * p.inv_gamma, m.rr, -q[0]);
 #pragma unroll
   for (int a = 0; a < DIM; ++a) {
     T ru = T(0);
 #pragma unroll
     for (int x = 0; x < DIM; ++x) {
-      ru -= ub[x] * g[1 + a][x];
-      const Coef<T>& gu = p.gu[a * 3 + x];
-      if (!gu.zero) ru -= (q[1 + x] + rr * ub[x]) * cval(gu, l);
+      ru = fma_t(-m.ub[x], g[1 + a][x], ru);
+      if (p.mean_terms & 2) ru = fma_t(-fma_t(rr, m.ub[x], q[1 + x]), m.gu[a][x], ru);
     }
-    ru -= g[P][a] * rbi;
-    r[1 + a] = ru;
+    r[1 + a] = fma_t(-g[P][a], m.rbi, ru);
   }
   {
     T rp = T(0);
-    const T pb = cval(p.pbar, l);
+    const T gpb = p.gamma * m.pb, gq = p.gamma * q[P];
 #pragma unroll
     for (int x = 0; x < DIM; ++x) {
-      rp -= ub[x] * g[P][x];
-      if (!p.gp[x].zero) rp -= q[1 + x] * cval(p.gp[x], l);
-      rp -= p.gamma * pb * g[1 + x][x];
-      const Coef<T>& gu = p.gu[x * 3 + x];
-      if (!gu.zero) rp -= p.gamma * q[P] * cval(gu, l);
+      rp = fma_t(-m.ub[x], g[P][x], rp);
+      if (p.mean_terms & 4) rp = fma_t(-q[1 + x], m.gp[x], rp);
+      rp = fma_t(-gpb, g[1 + x][x], rp);
+      if (p.mean_terms & 2) rp = fma_t(-gq, m.gu[x][x], rp);
     }
     r[P] = rp;
   }

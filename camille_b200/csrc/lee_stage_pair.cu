@@ -1,4 +1,4 @@
-// Fused RK stage for the compensated FP32 form on uniform-mean blocks, two points per thread
+// Fused RK stage for the compensated FP32 form on blocks without holes, two points per thread
 // (sm_100a).
 //
 // The same stage as k_stage_tma (lee_tma.cu): a CTA owns a 32 x 8 tile in (i, j) and marches
@@ -6,10 +6,17 @@
 // thread owns two neighbouring points along xi and computes them as a pair with the packed FP32
 // instructions of sm_100 (__ffma2_rn, __fadd2_rn, __fmul2_rn): derivatives, chain rule, the LEE
 // right-hand side (compute_RHS_linearized_Euler, src/solver/spatial_discretization.cpp:2053-2130,
-// uniform mean: every mean-gradient term vanishes), the Freund sponge and the compensated RK
+// of a uniform mean every mean-gradient term vanishes), the Freund sponge and the compensated RK
 // update (RungeKutta::integrate, src/solver/temporal_discretization.cpp:205-229) issue once per
 // pair, and shared and global memory move 8-byte pairs. Results are those of the one-point kernel
 // up to FP32 rounding order.
+//
+// With a non-uniform mean flow 21 coefficient pairs more are read per pair of points, without
+// branches (StageParams::mean), when the plane begins, so that they are in flight during the wait
+// and the derivatives. Held together with the inputs of the next plane they take up to 250
+// registers: two CTAs of 128 threads per SM. Bound by memory (220 bytes per point with all
+// coefficients fields: 47 us at 128 x 112 x 96); there 53 us per launch, the one-point kernel 134
+// with a branch per coefficient and 141 without (80 registers, spills).
 //
 // Every mbarrier wait is bounded (about one second); on expiry the CTA records the failure in the
 // device flag, waits (bounded) for its own copies in flight and returns.
@@ -21,7 +28,7 @@ namespace lee {
 namespace {
 
 template <int DIM, int TR>
-__global__ void __launch_bounds__(128, 3)
+__global__ void __launch_bounds__(128, (TR & kTrUniform) ? 3 : 2)
     k_stage_pair(const __grid_constant__ FieldMaps zm, const __grid_constant__ TmaStageParams<float> P) {
   using T = float;
   constexpr int H = kFdHalf, TX = kTileX, TY = kTileY, V = DIM + 2;
@@ -90,6 +97,8 @@ __global__ void __launch_bounds__(128, 3)
   auto plane = [&](int k, PairIn<DIM>& cur, PairIn<DIM>& nxt) -> bool {
     const unsigned lk = lij + nxy * (unsigned)k;
     if (active && k + 1 < k1) gather_pair<DIM, TR>(s, lk + nxy, nxt);
+    PairField<DIM> mean;  // in flight during the wait and the derivatives
+    if (!(TR & kTrUniform) && active) gather_mean_pair<DIM, TR>(s, lk, mean);
     bool failed = false;
     const int need = DIM == 3 ? min(phi, k + H) : 0;
     // `waited` stays at a plane whose wait gave up, so the drain below starts there
@@ -154,7 +163,7 @@ __global__ void __launch_bounds__(128, 3)
           D[v][DIM - 1] = dz;
         }
       }
-      pair_update<DIM, TR>(s, M, lk, i, j, k, src_ij0, D, q, cur);
+      pair_update<DIM, TR>(s, M, lk, i, j, k, src_ij0, D, q, cur, mean);
     }
     sk = sk + 1 == NS ? 0 : sk + 1;
     return true;
@@ -179,16 +188,20 @@ cudaError_t go_pair(const FieldMaps& z, const TmaStageParams<float>& p, int tile
   return cudaGetLastError();
 }
 
-// layout traits (JmField, Sponge; Uniform is required) and the stage kind
+// layout traits and the stage kind
 template <int DIM, int KIND>
 cudaError_t go_pair_layout(const FieldMaps& z, const TmaStageParams<float>& p, int tr, int tiles, int chunks,
                            cudaStream_t s) {
-  constexpr int B = kTrTma | kTrUniform | (KIND << kKindShift);
-  switch (tr & (kTrJmField | kTrSponge)) {
+  constexpr int B = kTrTma | (KIND << kKindShift), U = kTrUniform;
+  switch (tr & (kTrJmField | kTrSponge | kTrUniform)) {
     case 0: return go_pair<DIM, B>(z, p, tiles, chunks, s);
     case kTrJmField: return go_pair<DIM, B | kTrJmField>(z, p, tiles, chunks, s);
     case kTrSponge: return go_pair<DIM, B | kTrSponge>(z, p, tiles, chunks, s);
-    default: return go_pair<DIM, B | kTrJmField | kTrSponge>(z, p, tiles, chunks, s);
+    case kTrJmField | kTrSponge: return go_pair<DIM, B | kTrJmField | kTrSponge>(z, p, tiles, chunks, s);
+    case U: return go_pair<DIM, B | U>(z, p, tiles, chunks, s);
+    case U | kTrJmField: return go_pair<DIM, B | U | kTrJmField>(z, p, tiles, chunks, s);
+    case U | kTrSponge: return go_pair<DIM, B | U | kTrSponge>(z, p, tiles, chunks, s);
+    default: return go_pair<DIM, B | U | kTrJmField | kTrSponge>(z, p, tiles, chunks, s);
   }
 }
 
@@ -208,7 +221,7 @@ cudaError_t go_pair_kind(const FieldMaps& z, const TmaStageParams<float>& p, int
 }  // namespace
 
 bool stage_pair_applies(int traits, int px) {
-  return (traits & kTrTma) && (traits & kTrUniform) && ((traits >> kKindShift) & 7) != kKindRuntime && px % 2 == 0;
+  return (traits & kTrTma) && ((traits >> kKindShift) & 7) != kKindRuntime && px % 2 == 0;
 }
 
 cudaError_t launch_stage_pair(const FieldMaps& zin, const TmaStageParams<float>& p, int traits, int tiles, int chunks,

@@ -109,7 +109,7 @@ cudaError_t launch_adj_tma(const AdjMaps& m, const AdjTmaParams<T>& p, bool jm_f
                            cudaStream_t s);
 
 // The FP32 stage kernel with two points per thread (lee_stage_pair.cu): compensated form,
-// uniform mean flow, TMA blocks of an even row pitch, a fixed stage kind.
+// TMA blocks without holes of an even row pitch, a fixed stage kind.
 bool stage_pair_applies(int traits, int px);
 cudaError_t launch_stage_pair(const FieldMaps& zin, const TmaStageParams<float>& p, int traits, int tiles, int chunks,
                               cudaStream_t s);
