@@ -14,6 +14,8 @@
 namespace lee {
 namespace {
 
+constexpr int kWideHalf = 5;  // half-width of the 11-point difference
+
 // Operator value at one point: the interior stencil, or a closure row selected by
 // position along the line or by the precomputed code (src/solver/spatial_discretization.cpp:1094-1149
 // and the hole closures of :1656-1745).
@@ -73,6 +75,75 @@ __global__ void __launch_bounds__(256) k_stage(StageParams<T> p) {
     q[v] = p.zin[v][l];
   }
   rhs_update<T, DIM, COMP, kTrGeneric>(p, l, i, j, k, D, q, in, mean);
+}
+
+// k_stage for the 11-point difference on a block without closure codes: the half-width is known at
+// compile time, and a point's window along a line is its 11 points moved into the line, with the
+// weights of its closure class (0 interior, 1..5 left, 6..10 right rows) from shared memory, so
+// that boundary and interior points of a warp run the same instructions. Bound by the 165 cached
+// loads per point (FP64: 32 us of L1 bandwidth at 96^3); 128 threads, five CTAs per SM for the
+// uniform mean flow: 75 us per launch at 96^3 FP64, with four CTAs 80, six 78, and 88 with 256
+// threads (any shape of tile in j and k is within 3 %); k_stage, whose loops over the operator run
+// to a length read at run time, 213.
+template <typename T, int DIM, bool COMP, int TR>
+__global__ void __launch_bounds__(128, (TR & kTrUniform) ? 5 : 4) k_stage_wide(const __grid_constant__ StageParams<T> p) {
+  constexpr int V = DIM + 2, W = 2 * kWideHalf + 1, NC = 1 + 2 * kWideHalf;
+  __shared__ T w[NC][W];
+  const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+  for (int q = tid; q < NC * W; q += blockDim.x * blockDim.y * blockDim.z) {
+    const int c = q / W, o = q % W;
+    double x = 0.0;
+    if (c == 0) x = p.fd.c[o];
+    else if (c <= kWideHalf) x = o < p.fd.S ? p.fd.B[c - 1][o] : 0.0;
+    else x = W - 1 - o < p.fd.S ? p.fd.mfac * p.fd.B[c - 1 - kWideHalf][W - 1 - o] : 0.0;
+    w[c][o] = (T)x;
+  }
+  __syncthreads();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int k = blockIdx.z * blockDim.z + threadIdx.z;
+  if (i >= p.nx || j >= p.ny || k >= p.nz) return;
+  const long long nxy = (long long)p.px * p.ny;
+  const long long l = i + (long long)p.px * j + nxy * k;
+  const int pos[3] = {i, j, k};
+  const int nn[3] = {p.nx, p.ny, p.nz};
+  const long long sd[3] = {1, p.px, nxy};
+  T D[V][DIM], q[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) q[v] = __ldg(p.zin[v] + l);
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    const int a = min(max(pos[d] - kWideHalf, 0), nn[d] - W);
+    const int r = nn[d] - 1 - pos[d];
+    const T* wc = w[pos[d] < kWideHalf ? 1 + pos[d] : r < kWideHalf ? 1 + kWideHalf + r : 0];
+    const long long l0 = l + (a - pos[d]) * sd[d];
+    T wd[W];
+#pragma unroll
+    for (int o = 0; o < W; ++o) wd[o] = wc[o];
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      const T* f = p.zin[v] + l0;
+      T t = T(0);
+#pragma unroll
+      for (int o = 0; o < W; ++o) t = fma_t(wd[o], __ldg(f + o * sd[d]), t);
+      D[v][d] = t;
+    }
+  }
+  PointIn<T, DIM> in;
+  gather<T, DIM, COMP, TR>(p, l, in);
+  PointMean<T, DIM> mean;
+  if (!(TR & kTrUniform)) gather_mean<T, DIM, TR>(p, l, mean);
+  rhs_update<T, DIM, COMP, TR>(p, l, i, j, k, D, q, in, mean);
+}
+
+template <typename T, int DIM, bool COMP>
+cudaError_t go_wide(const StageParams<T>& p, cudaStream_t s) {
+  const dim3 blk(32, 4, 1), grd((p.nx + 31) / 32, (p.ny + 3) / 4, p.nz);
+  bool uniform = p.mean_terms == 0;
+  for (int q = kMeanUb; q <= kMeanPb; ++q) uniform &= p.mean_mask[q] == 0;
+  if (uniform) k_stage_wide<T, DIM, COMP, kTrGeneric | kTrUniform><<<grd, blk, 0, s>>>(p);
+  else k_stage_wide<T, DIM, COMP, kTrGeneric><<<grd, blk, 0, s>>>(p);
+  return cudaGetLastError();
 }
 
 // One direction of spatial::apply_filter (src/solver/spatial_discretization.cpp:2191-2246).
@@ -222,6 +293,10 @@ cudaError_t launch_scalar_stage(const ScalarParams<T>& p, int comp, cudaStream_t
 
 template <typename T>
 cudaError_t launch_stage(const StageParams<T>& p, int comp, cudaStream_t s) {
+  if (p.fd.h == kWideHalf && !p.code[0]) {  // (lines have at least 2 h + 1 points, checked at setup)
+    if (p.dim == 2) return comp ? go_wide<T, 2, true>(p, s) : go_wide<T, 2, false>(p, s);
+    return comp ? go_wide<T, 3, true>(p, s) : go_wide<T, 3, false>(p, s);
+  }
   dim3 blk(32, 8, 1);
   dim3 grd((p.nx + 31) / 32, (p.ny + 7) / 8, p.nz);
   if (p.dim == 2) {

@@ -1,6 +1,7 @@
 """Stage kernels with a non-uniform mean flow: which of the entropy, velocity and pressure gradients
 are present, constant and varying coefficients, curvilinear metrics, aligned and ragged rows, single
-planes of a chunk.
+planes of a chunk; and the 11-point difference, whose kernel moves each point's window into the line
+(lines of 11 points, the shortest it takes, and up).
 
 Tolerances: FP64 1e-12. In FP32 a right-hand side is a sum of up to 40 rounded terms of the size of
 the result (the state is noise, nothing cancels): sqrt(40) * 6e-8 = 4e-7, so 1e-6."""
@@ -65,3 +66,14 @@ def test_the_two_point_kernel_stays_a_choice_of_uniform_blocks(product_lib):
     with pytest.raises(api.LeeError):
         api.Solver(product_lib, _block(32, 16, 9, "su"), precision=api.FP32_COMPENSATED, stage_kernel=2)
     api.Solver(product_lib, _block(32, 16, 9, "su"), precision=api.FP32_COMPENSATED, stage_kernel=1).advance(1, 0.2)
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+@pytest.mark.parametrize("terms", ["", "sup"])
+@pytest.mark.parametrize("nx,ny,nz", [(11, 11, 11), (12, 13, 17), (33, 11, 15), (34, 15, 11), (40, 21, 1), (11, 37, 1)])
+def test_eleven_points_match_oracle(product_lib, oracle_lib, nx, ny, nz, terms, precision):
+    case = _block(nx, ny, nz, terms, bend=0.2, sponge=3 if min(nx, ny) >= 12 else 0)
+    case.fd_scheme, case.filter_scheme, case.filter_strength = "FDO11P", "SFO11P", 0.2
+    if terms:
+        case.rk = "RUNGE_KUTTA2"
+    _check(case, product_lib, oracle_lib, precision)
