@@ -199,7 +199,9 @@ struct lee_ctx {
   unsigned long long wait_ns = kDefaultWaitNs;  // limit of the kernels' waits on staged data
   int finite_every = 0;          // lee_set_finite_check: steps between checks (0: end of each advance, -1: off)
   double* d_report = nullptr;  // -min and max of the five state slots (lee_state_minmax)
-  double* d_staging = nullptr;  // FP64 field of compensated uploads and downloads
+  double* d_staging = nullptr;  // FP64 fields of converting uploads and downloads
+  long long staging_points = 0;
+  double* d_cfl = nullptr;      // CFL maximum per block
   // overset maps (host copies, then device arrays from lee_prepare)
   struct {
     int n = 0, W = 1, w[3] = {1, 1, 1};

@@ -483,9 +483,12 @@ cudaError_t setup_minmax(int n, const double* f, double* d_out2, cudaStream_t s)
 // over the nx points of each of `rows` rows px points apart
 cudaError_t setup_state_minmax(long long rows, int nx, int px, const void* y, const void* e, bool fp32, double* d_out2,
                                cudaStream_t s);
-cudaError_t setup_cfl(int n, int dim, const double* const* met, const double* jac, const double* const* ubar,
-                      const double* pbar, const double* sbar, const int* iblank, double gamma, double dt,
-                      double* d_max, cudaStream_t s);
+// Fields of the CFL maximum.
+struct CflFields {
+  const double *met[9], *ub[3], *jac, *pbar, *sbar;
+  const int* iblank;
+};
+cudaError_t setup_cfl(int n, int dim, const CflFields& f, double gamma, double dt, double* d_max, cudaStream_t s);
 cudaError_t setup_rho_ratio(int n, int V, double gamma, const double* sv, const double* p, const double* pbar,
                             double* out, cudaStream_t s);
 cudaError_t setup_monopole_g(int nx, int ny, const double* const* xyz, const int lo[3], const int hi[3],

@@ -236,34 +236,32 @@ __global__ void k_state_minmax(long long rows, int nx, int px, const T* y, const
 
 // temporal::compute_CFL (src/solver/temporal_discretization.cpp:397-450), including the
 // convective term's truncation to int (abs(double) resolving to int abs(int) at :425).
-__global__ void k_cfl(long long n, int dim, const double* const* met, const double* jac, const double* const* ub,
-                      const double* pbar, const double* sbar, const int* iblank, double gamma, double dt,
-                      double* d_max) {
+__global__ void k_cfl(long long n, int dim, CflFields f, double gamma, double dt, double* d_max) {
   __shared__ double sm[kThreads];
   double best = -1e300;
   for (long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x; l < n; l += (long long)gridDim.x * blockDim.x) {
-    if (iblank && iblank[l] != 0) continue;
+    if (f.iblank && f.iblank[l] != 0) continue;
     double vc[3] = {0, 0, 0};
     for (int a = 0; a < dim; ++a) {
       vc[a] = 0.0;
-      for (int q = 0; q < dim; ++q) vc[a] += met[a * 3 + q][l] * ub[q][l];
+      for (int q = 0; q < dim; ++q) vc[a] += f.met[a * 3 + q][l] * f.ub[q][l];
     }
     double cfl = 0.0;
     for (int a = 0; a < dim; ++a)
       for (int q = 0; q < dim; ++q) {
-        int t = (int)(vc[a] * met[a * 3 + q][l]);
+        int t = (int)(vc[a] * f.met[a * 3 + q][l]);
         cfl += (double)(t < 0 ? -t : t);
       }
     double fac = 0.0;
     for (int a = 0; a < dim; ++a)
-      for (int q = 0; q < dim; ++q) fac += met[a * 3 + q][l] * met[a * 3 + q][l];
+      for (int q = 0; q < dim; ++q) fac += f.met[a * 3 + q][l] * f.met[a * 3 + q][l];
     // State::compute_auxiliary_variables_linear_Euler (src/core/state.cpp:701-736)
     double g = gamma, gi = 1.0 / g, gg = g / (g - 1.0);
-    double rhobar = pow(g * pbar[l], gi) * exp(-sbar[l]);
-    double Tbar = pbar[l] * gg * (1.0 / rhobar);
+    double rhobar = pow(g * f.pbar[l], gi) * exp(-f.sbar[l]);
+    double Tbar = f.pbar[l] * gg * (1.0 / rhobar);
     double sos = sqrt((gamma - 1.0) * Tbar);
     cfl += sos * sqrt(fac);
-    cfl *= dt * jac[l];
+    cfl *= dt * f.jac[l];
     best = cfl > best ? cfl : best;
   }
   sm[threadIdx.x] = best;
@@ -368,10 +366,8 @@ cudaError_t setup_state_minmax(long long rows, int nx, int px, const void* y, co
   return cudaGetLastError();
 }
 
-cudaError_t setup_cfl(int n, int dim, const double* const* met, const double* jac, const double* const* ubar,
-                      const double* pbar, const double* sbar, const int* iblank, double gamma, double dt,
-                      double* d_max, cudaStream_t s) {
-  k_cfl<<<grid_for(n), kThreads, 0, s>>>(n, dim, met, jac, ubar, pbar, sbar, iblank, gamma, dt, d_max);
+cudaError_t setup_cfl(int n, int dim, const CflFields& f, double gamma, double dt, double* d_max, cudaStream_t s) {
+  k_cfl<<<grid_for(n), kThreads, 0, s>>>(n, dim, f, gamma, dt, d_max);
   return cudaGetLastError();
 }
 
