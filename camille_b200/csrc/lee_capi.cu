@@ -227,7 +227,7 @@ void lee_destroy(lee_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->cfg.device);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  if (c->graph.exec) cudaGraphExecDestroy(c->graph.exec);
+  drop_graphs(c);
   for (auto e : c->ev_pool) cudaEventDestroy(e);
   if (c->adj.rev) {
     cudaStreamSynchronize(c->adj.rev);

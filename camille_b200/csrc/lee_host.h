@@ -150,6 +150,13 @@ using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
 
 }  // namespace lee
 
+// Captured steps, ready to launch.
+struct StepGraph {
+  cudaGraphExec_t exec = nullptr;
+  int steps = 0;                                                    // per replay
+  long long launches = 0, stage_launches = 0, filter_launches = 0;  // per replay
+};
+
 struct lee_ctx {
   lee_config cfg;
   int V = 0;
@@ -213,15 +220,14 @@ struct lee_ctx {
     long long *d_rl = nullptr, *d_dl = nullptr;
     double *d_wt = nullptr, *d_buf = nullptr;
   } ovs;
-  // replayed step graph: a few steps captured once (until the buffer roles repeat) and
-  // launched as one graph; keyed by dt, precision and the buffer layout it was captured on
+  // replayed step graphs: a few steps captured once (until the buffer roles repeat) and
+  // launched as one graph, and for long calls several such periods in one; keyed by dt, precision
+  // and the buffer layout they were captured on
   struct {
     bool enabled = true;
-    cudaGraphExec_t exec = nullptr;
+    StepGraph one, many;
     std::vector<double> dts;       // the time step of every block
-    int steps = 0;                 // steps per replay
     std::vector<void*> layout;
-    long long launches = 0, stage_launches = 0, filter_launches = 0;  // per replay
     void* d_amp = nullptr;         // monopole amplitudes, [step][stage], working precision
     size_t amp_cap = 0;            // entries
     int* d_ctr = nullptr;          // steps of the current chunk done so far
@@ -423,7 +429,8 @@ Clocks save_clocks(const lee_ctx* c);
 void restore_clocks(lee_ctx* c, const Clocks& k);
 void set_clock(lee_ctx* c, double t, int step);
 template <typename T>
-int capture_steps(lee_ctx* c, const std::vector<double>& dts);
+int capture_steps(lee_ctx* c, const std::vector<double>& dts, int periods, StepGraph* out);
+void drop_graphs(lee_ctx* c);
 template <typename T>
 int advance_impl(lee_ctx* c, int nsteps, const std::vector<double>& dts);
 int advance_timed(lee_ctx* c, int nsteps, const std::vector<double>& dts);

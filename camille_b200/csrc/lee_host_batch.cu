@@ -385,10 +385,7 @@ int lee_set_batch_shapes(lee_ctx* c, int stage_shape, int filter_shape) {
                            : batch_filter_occupancy<double>(filter_shape, 0);
   bt.sgrid = std::min(bt.nst, nsm * occs);
   bt.fgrid = std::min(4 * bt.nft, nsm * occf);
-  if (c->graph.exec) {  // captured launches name the old work lists
-    cudaGraphExecDestroy(c->graph.exec);
-    c->graph.exec = nullptr;
-  }
+  drop_graphs(c);  // captured launches name the old work lists
   return LEE_OK;
 }
 
@@ -408,10 +405,7 @@ int lee_set_batch_persistent(lee_ctx* c, int shape) {
     if (!bt.d_gbar && (rc = dalloc(c, &bt.d_gbar, 2))) return rc;
   }
   bt.pshape = shape;
-  if (c->graph.exec) {  // captured launches name the old schedule
-    cudaGraphExecDestroy(c->graph.exec);
-    c->graph.exec = nullptr;
-  }
+  drop_graphs(c);  // captured launches name the old schedule
   return LEE_OK;
 }
 

@@ -165,6 +165,7 @@ int launch_stage_any(lee_ctx* c, BlockData& b, const StageParams<T>& p, void* co
   if (b.plane_stage && kind != kKindRuntime && kind != kKindLastIncrement) {
     PlaneStage<T> pp;
     pp.s = p;
+    pp.overlap = c->blk.size() == 1 && !c->timing;
     for (int a = 0; a < 6; ++a)
       for (int o = 0; o < 5; ++o) pp.w[a][o] = (T)c->wst[a][o];
     CK(launch_plane_stage<T>(pp, tr, c->stream));
@@ -221,6 +222,7 @@ int launch_filter_fused(lee_ctx* c, BlockData& b, void* const* in, void* const* 
     pf.ny = b.ny;
     pf.px = b.px;
     pf.rows = plane_filter_rows(b, c->V);
+    pf.overlap = c->blk.size() == 1 && !c->timing;
     if (b.has_holes) {
       pf.code[0] = b.d_tcode_flt[0];
       pf.code[1] = b.d_tcode_flt[1];

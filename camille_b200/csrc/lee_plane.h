@@ -35,6 +35,7 @@ template <typename T>
 struct PlaneStage {
   StageParams<T> s;
   T w[6][5];
+  int overlap;  // launch while the stream's previous kernel still runs (the kernel waits for its end)
 };
 
 // One field of a filter launch: the pre-filter values, their rounding error (compensated), the
@@ -57,6 +58,7 @@ struct PlaneFilter {
   const int* iblank;
   T blend;
   PlaneFilterField<T> f[kMaxVars];
+  int overlap;  // as in PlaneStage
 };
 
 // traits: the block's layout traits and the stage's kind (not the increment kind)
