@@ -110,7 +110,7 @@ struct BlockData {
   int stage_chunk = 0, filter_chunk = 0;
   int filter_ry = 1;                  // rows per thread row of the scalar fused filter (1 or 2)
   int filter_form = 0;                // lee_set_filter_form where the block can run it, else 0 (timed)
-  bool filter_pair_ok = false;        // the two-point compensated filter (lee_filter_pair.cu) applies
+  bool filter_pair_ok = false;        // the two-row filter (lee_filter_pair.cu) applies
   bool filter_pair = false;           // ... and runs the block's fused filter (form 3)
   int ptiles_x = 0, ptiles_y = 0;     // its tiles
   int tfilter_ry = 1, tfilter_chunk = 0;  // the scalar form and chunk of the adjoint's transposed filter

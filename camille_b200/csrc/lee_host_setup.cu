@@ -476,15 +476,15 @@ int lee_prepare(lee_ctx* c) {
       if (ok) b.filter_px = c->filter_kernel;
     }
     b.filter_ry = 1;
-    // the two-point form: compensated FP32, 3-D, no holes, even nxi, the scalar kernel's place
-    b.filter_pair_ok = b.tma_filter && c->comp && c->cfg.num_dim == 3 && !b.has_holes && b.px % 2 == 0 &&
+    // the two-row form: 3-D, no holes, the scalar kernel's place (by number: the compensated form's)
+    b.filter_pair_ok = b.tma_filter && c->cfg.num_dim == 3 && !b.has_holes && b.px % 2 == 0 &&
                        b.filter_px == 0 && filter_pair_half_width(c->hf);
     b.filter_pair = false;
     b.filter_form = 0;
     if (c->filter_form > 0 && b.tma_filter) {
       // the two-row and two-point forms take neither holes nor the vector kernel's groups
       const bool ok = c->filter_form == 1 || (c->filter_form == 2 && b.filter_px == 0 && !b.has_holes) ||
-                      (c->filter_form == 3 && b.filter_pair_ok);
+                      (c->filter_form == 3 && b.filter_pair_ok && c->comp);
       if (!ok && b.px == b.nx)
         return fail(c, LEE_ERR_UNSUPPORTED, "filter form %d is not available for block %d", c->filter_form,
                     (int)(&b - c->blk.data()));
