@@ -261,8 +261,8 @@ int lee_advance_blocks(lee_ctx *ctx, int nsteps, const double *dt);
 /* The FIX_CFL time step of every block on its own (dt[b], as lee_compute_dt would give for a
  * context holding block b alone). */
 int lee_compute_dt_blocks(lee_ctx *ctx, double cfl, double *dt);
-/* Override the batched launches' work-item shapes that lee_prepare picked by timing (index
- * 0..6; lee_info reports the strip of each): every shape gives the same results. */
+/* Run a batch's strip kernels with these work-item shapes (index 0..6; lee_info reports the strip
+ * of each) instead of the default tiles: every shape gives the same results. */
 int lee_set_batch_shapes(lee_ctx *ctx, int stage_shape, int filter_shape);
 /* One launch per batched step (no reference counterpart; the same bits as the per-phase
  * launches): shape 0..4 (a work-item shape with one column per stage thread; lee_info's tiles
