@@ -225,6 +225,7 @@ struct lee_ctx {
   // and the buffer layout they were captured on
   struct {
     bool enabled = true;
+    bool capturing = false;        // capture_steps is recording: no launch may read host memory later
     StepGraph one, many;
     std::vector<double> dts;       // the time step of every block
     std::vector<void*> layout;
@@ -419,7 +420,7 @@ int batch_setup(lee_ctx* c);
 template <typename T>
 int batch_refresh(lee_ctx* c);
 template <typename T>
-int batch_step(lee_ctx* c, const std::vector<double>& dts, bool graph);
+int batch_step(lee_ctx* c, const std::vector<double>& dts, bool capturing);
 template <typename T>
 int step_impl(lee_ctx* c, const std::vector<double>& dts, const T* amp_tab, const double* t_tab, const int* ctr);
 std::vector<void*> layout_of(lee_ctx* c);

@@ -298,14 +298,16 @@ int batch_refresh(lee_ctx* c) {
   return LEE_OK;
 }
 
-// One batched step (see step_impl): ns stage launches and one filter launch for every block.
+// One batched step (see step_impl): ns stage launches and one filter launch for every block. A
+// captured step reads the parameters that advance_impl placed in d_prm_graph, with or without
+// sources: a copy from this frame, recorded into the graph, would read the frame at each replay.
 template <typename T>
-int batch_step(lee_ctx* c, const std::vector<double>& dts, bool graph) {
+int batch_step(lee_ctx* c, const std::vector<double>& dts, bool capturing) {
   auto& bt = c->batch;
   const Tableau tb = tableau(c->cfg.rk_scheme);
   const int nbk = (int)c->blk.size();
   const void* prm = bt.d_prm_graph;
-  if (!graph) {
+  if (!capturing) {
     std::vector<StageParams<T>> pr = batch_params<T>(c, dts, false, 0);
     CK(cudaMemcpyAsync(bt.d_prm_direct, pr.data(), pr.size() * sizeof(pr[0]), cudaMemcpyHostToDevice, c->stream));
     prm = bt.d_prm_direct;
@@ -354,8 +356,8 @@ template int batch_setup<float>(lee_ctx* c);
 template int batch_setup<double>(lee_ctx* c);
 template int batch_refresh<float>(lee_ctx* c);
 template int batch_refresh<double>(lee_ctx* c);
-template int batch_step<float>(lee_ctx* c, const std::vector<double>& dts, bool graph);
-template int batch_step<double>(lee_ctx* c, const std::vector<double>& dts, bool graph);
+template int batch_step<float>(lee_ctx* c, const std::vector<double>& dts, bool capturing);
+template int batch_step<double>(lee_ctx* c, const std::vector<double>& dts, bool capturing);
 
 }  // namespace lee
 

@@ -56,7 +56,7 @@ int step_impl(lee_ctx* c, const std::vector<double>& dts, const T* amp_tab, cons
     c->time = c->blk[0].time;
     c->step = c->blk[0].step;
     if (c->batch.active) {
-      int rc = batch_step<T>(c, dts, ctr != nullptr);
+      int rc = batch_step<T>(c, dts, c->graph.capturing);
       if (rc) return rc;
       return trace_step<T>(c, ctr);
     }
@@ -313,6 +313,7 @@ int capture_steps(lee_ctx* c, const std::vector<double>& dts, int periods, StepG
   const bool src = c->src_kind != LEE_SOURCE_NONE;
   const bool tick = src || c->adj.trace_on || c->wave_time;
   CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed));
+  g.capturing = true;
   int rc = LEE_OK, steps = 0, done = 0;
   for (; steps < 4 * periods;) {
     rc = step_impl<T>(c, dts, src ? (const T*)g.d_amp : nullptr, c->wave_time ? g.d_ttab : nullptr,
@@ -325,6 +326,7 @@ int capture_steps(lee_ctx* c, const std::vector<double>& dts, int periods, StepG
     ++steps;
     if (layout_of(c) == start && ++done == periods) break;
   }
+  g.capturing = false;
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
   const bool repeat = rc == LEE_OK && layout_of(c) == start;
