@@ -646,12 +646,18 @@ __global__ void __launch_bounds__(32 * kPlaneWarps, sizeof(T) == 4 ? 3 : 2)
   const int v = blockIdx.y, tid = (int)threadIdx.y * 32 + (int)threadIdx.x;
   const int t0 = (int)blockIdx.x * per, t1 = min(t0 + per, ntiles);
   int issued = t0;  // thread 0: tiles whose copies are under way
+  int acquired = -1;  // ... and the block whose map it has acquired
   auto issue_upto = [&](int last) {
     for (; issued < min(t1, last); ++issued) {
       const int4 t = __ldg(tiles + issued);
       const int q = (issued - t0) % NS;
+      const CUtensorMap* map = maps + t.x * 4 + v;
+      if (t.x != acquired) {
+        acquire_map(map);
+        acquired = t.x;
+      }
       mbar_expect_tx(&bar[q], (unsigned)(sizeof(T) * B::FB));
-      tma_load_3d(ring + q * B::FB, maps + t.x * 4 + v, t.y - B::HX, t.z - 4, 0, &bar[q]);
+      tma_load_3d(ring + q * B::FB, map, t.y - B::HX, t.z - 4, 0, &bar[q]);
     }
   };
   if (tid == 0) {

@@ -67,6 +67,14 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
       : "memory");
 }
 
+// A tensor map in global memory may have been rewritten by the host since this SM last used the
+// address: the map's proxy must acquire the new value, in each block before its first copy. (Maps
+// passed as __grid_constant__ parameters need none.)
+__device__ __forceinline__ void acquire_map(const CUtensorMap* map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(reinterpret_cast<unsigned long long>(map))
+               : "memory");
+}
+
 template <int N, typename F, int... I>
 __device__ __forceinline__ void static_for_impl(F&& f, std::integer_sequence<int, I...>) {
   (f(std::integral_constant<int, I>{}), ...);

@@ -67,3 +67,33 @@ def test_same_bits_after_filter_calls_and_other_shapes(product_lib, precision):
         assert product_lib.set_batch_shapes(s.ctx, 1, 3) == api.LEE_OK
         s.advance_blocks(133, dts)
     _same(a, b, case)
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+def test_maps_of_later_buffers_and_contexts(product_lib, precision):
+    """The batched filter's maps are rewritten in place when buffers swap, and a later context's may
+    land where a destroyed one's were: what is copied is always the present buffer."""
+    want = None
+    for turn in range(4):
+        case = _batch(count=5 if turn % 2 == 0 else 7)
+        s = api.Solver(product_lib, case, precision=precision)
+        dts = 0.5 * s.compute_dt_blocks()
+        for _ in range(3):
+            s.advance_blocks(2, dts)
+            s.apply_filter()
+        s.advance_blocks(3, dts)
+        got = [s.download(q)[0] for q in range(len(case.blocks))]
+        s.close()
+        if turn == 0:
+            want = got
+        elif turn == 2:
+            for a, b in zip(got, want):
+                np.testing.assert_array_equal(a, b)
+        t = api.Solver(product_lib, case, precision=precision, batching=False)
+        for _ in range(3):
+            t.advance_blocks(2, dts)
+            t.apply_filter()
+        t.advance_blocks(3, dts)
+        tol = 1e-12 if precision == api.FP64 else 1e-6
+        assert all(api.rel_l2(g, t.download(q)[0]) <= tol for q, g in enumerate(got))
+        t.close()
