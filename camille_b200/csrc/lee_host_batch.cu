@@ -151,7 +151,7 @@ int plane_batch_maps(lee_ctx* c) {
     int rc = encode_maps(c, b, c->comp ? b.zb[(ns - 1) % 2] : b.acc, 4, bx, by, &m[q * 4]);
     if (rc) return rc;
   }
-  CK(cudaMemcpy(c->batch.d_maps, m.data(), m.size() * sizeof(m[0]), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(c->batch.d_maps, m.data(), m.size() * sizeof(m[0]), cudaMemcpyHostToDevice, c->stream));
   return LEE_OK;
 }
 
@@ -198,8 +198,8 @@ int batch_setup(lee_ctx* c) {
   int4* d_t = nullptr;
   CK(cudaMalloc(&d_pr, pr.size() * sizeof(pr[0])));
   CK(cudaMalloc(&d_fs, fs.size() * sizeof(fs[0])));
-  CK(cudaMemcpy(d_pr, pr.data(), pr.size() * sizeof(pr[0]), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(d_fs, fs.data(), fs.size() * sizeof(fs[0]), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(d_pr, pr.data(), pr.size() * sizeof(pr[0]), cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(d_fs, fs.data(), fs.size() * sizeof(fs[0]), cudaMemcpyHostToDevice, c->stream));
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->cfg.device);
   cudaEvent_t e0, e1;
@@ -210,7 +210,7 @@ int batch_setup(lee_ctx* c) {
   for (int shape = 0; shape < kBatchShapes; ++shape) {
     std::vector<int4> t = batch_tiles(c, shape);
     CK(cudaMalloc(&d_t, t.size() * sizeof(int4)));
-    CK(cudaMemcpy(d_t, t.data(), t.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(d_t, t.data(), t.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
     const int nt = (int)t.size();
     const int gs = std::min(nt, nsm * batch_stage_occupancy<T>(shape, c->comp ? 1 : 0));
     // (the filter's CTAs each take a share of the items for some of the four fields)
@@ -249,8 +249,8 @@ int batch_setup(lee_ctx* c) {
   CK(cudaFree(d_pr));
   CK(cudaFree(d_fs));
   if ((rc = dalloc(c, &bt.d_stiles, tiles_s.size())) || (rc = dalloc(c, &bt.d_ftiles, tiles_f.size()))) return rc;
-  CK(cudaMemcpy(bt.d_stiles, tiles_s.data(), tiles_s.size() * sizeof(int4), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(bt.d_ftiles, tiles_f.data(), tiles_f.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(bt.d_stiles, tiles_s.data(), tiles_s.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(bt.d_ftiles, tiles_f.data(), tiles_f.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
   bt.nst = (int)tiles_s.size();
   bt.nft = (int)tiles_f.size();
   // the direct kernels serve every batch whose rows are 16-byte multiples (the row pitch's doing);
@@ -264,8 +264,8 @@ int batch_setup(lee_ctx* c) {
   if (bt.plane) {
     const std::vector<int4> ps = plane_tiles(c, kPlaneBatchTall), pf = plane_tiles(c, kPlaneWarps * kPlaneBatchRows);
     if ((rc = dalloc(c, &bt.d_pstiles, ps.size())) || (rc = dalloc(c, &bt.d_pftiles, pf.size()))) return rc;
-    CK(cudaMemcpy(bt.d_pstiles, ps.data(), ps.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(bt.d_pftiles, pf.data(), pf.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(bt.d_pstiles, ps.data(), ps.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(bt.d_pftiles, pf.data(), pf.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
     if ((rc = dalloc(c, &bt.d_maps, c->blk.size() * 4))) return rc;
     bt.npst = (int)ps.size();
     bt.npft = (int)pf.size();
@@ -291,7 +291,7 @@ int batch_refresh(lee_ctx* c) {
   if (roles == bt.roles) return LEE_OK;
   std::vector<BatchFilterInst<T>> fi = batch_filter_inst<T>(c, false);
   CK(cudaStreamSynchronize(c->stream));  // steps under way read the old operands
-  CK(cudaMemcpy(bt.d_finst, fi.data(), fi.size() * sizeof(fi[0]), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(bt.d_finst, fi.data(), fi.size() * sizeof(fi[0]), cudaMemcpyHostToDevice, c->stream));
   if (bt.plane)
     if (int rc = plane_batch_maps<T>(c)) return rc;
   bt.roles.swap(roles);
@@ -375,8 +375,8 @@ int lee_set_batch_shapes(lee_ctx* c, int stage_shape, int filter_shape) {
   const std::vector<int4> ts = batch_tiles(c, stage_shape), tf = batch_tiles(c, filter_shape);
   int rc;
   if ((rc = dalloc(c, &bt.d_stiles, ts.size())) || (rc = dalloc(c, &bt.d_ftiles, tf.size()))) return rc;
-  CK(cudaMemcpy(bt.d_stiles, ts.data(), ts.size() * sizeof(int4), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(bt.d_ftiles, tf.data(), tf.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(bt.d_stiles, ts.data(), ts.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(bt.d_ftiles, tf.data(), tf.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
   bt.nst = (int)ts.size();
   bt.nft = (int)tf.size();
   bt.sshape = stage_shape;
@@ -402,7 +402,7 @@ int lee_set_batch_persistent(lee_ctx* c, int shape) {
   if (shape >= 0) {
     const std::vector<int4> t = batch_tiles(c, shape);
     if ((rc = dalloc(c, &bt.d_ptiles, t.size()))) return rc;
-    CK(cudaMemcpy(bt.d_ptiles, t.data(), t.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(bt.d_ptiles, t.data(), t.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
     bt.npt = (int)t.size();
     if (!bt.d_gbar && (rc = dalloc(c, &bt.d_gbar, 2))) return rc;
   }

@@ -414,7 +414,7 @@ int advance_impl(lee_ctx* c, int nsteps, const std::vector<double>& dts) {
     if (c->batch.active) {
       // the stage parameters the captured batched launches read (amplitudes from the table)
       std::vector<StageParams<T>> pr = batch_params<T>(c, dts, true, 0);
-      CK(cudaMemcpy(c->batch.d_prm_graph, pr.data(), pr.size() * sizeof(pr[0]), cudaMemcpyHostToDevice));
+      CK(cudaMemcpyAsync(c->batch.d_prm_graph, pr.data(), pr.size() * sizeof(pr[0]), cudaMemcpyHostToDevice, c->stream));
       c->batch.graph_dts = dts;
     }
     int rc = capture_steps<T>(c, dts, 1, &g.one);
