@@ -280,12 +280,8 @@ __global__ void __launch_bounds__(256) k_adj_tma(const __grid_constant__ AdjMaps
 template <typename T, bool JMF>
 cudaError_t go_adj_tma(const AdjMaps& m, const AdjTmaParams<T>& p, int tiles, int chunks, cudaStream_t s) {
   using G = AGeo<T>;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_adj_tma<T, JMF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::BYTES);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static PerDevice smem;
+  if (const cudaError_t e = allow_smem(smem, k_adj_tma<T, JMF>, G::BYTES); e != cudaSuccess) return e;
   k_adj_tma<T, JMF><<<dim3(tiles, chunks), 256, G::BYTES, s>>>(m, p);
   return cudaGetLastError();
 }

@@ -444,13 +444,8 @@ __global__ void __launch_bounds__(256, PX * sizeof(T) == 16 ? 2 : 3)
 template <typename T, int DIM, bool COMP, int HF, int PX>
 cudaError_t go_filter_vec(const FieldMaps& in, const TmaFilterParams<T>& p, int tiles, int chunks, cudaStream_t s) {
   using G = FGeo<T, DIM, COMP, HF, PX>;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_filter_vec<T, DIM, COMP, HF, PX>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::BYTES);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static PerDevice smem;
+  if (const cudaError_t e = allow_smem(smem, k_filter_vec<T, DIM, COMP, HF, PX>, G::BYTES); e != cudaSuccess) return e;
   k_filter_vec<T, DIM, COMP, HF, PX><<<dim3(tiles, chunks, p.V), 256, G::BYTES, s>>>(in, p);
   return cudaGetLastError();
 }

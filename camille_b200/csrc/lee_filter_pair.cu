@@ -368,13 +368,8 @@ template <typename T, int HF, bool COMP>
 cudaError_t go_filter_pair(const FieldMaps& in, const TmaFilterParams<T>& p, int tiles, int chunks,
                            cudaStream_t s) {
   const size_t bytes = PairGeo<T, HF>::bytes(COMP);
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e =
-        cudaFuncSetAttribute(k_filter_pair<T, HF, COMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static PerDevice smem;
+  if (const cudaError_t e = allow_smem(smem, k_filter_pair<T, HF, COMP>, bytes); e != cudaSuccess) return e;
   k_filter_pair<T, HF, COMP><<<dim3(tiles, chunks, p.V), 32 * kPairWarps, bytes, s>>>(in, p);
   return cudaGetLastError();
 }

@@ -715,12 +715,12 @@ cudaError_t go_stage_layout(const PlaneStage<T>& p, int traits, cudaStream_t s) 
   }
 }
 
-// CTAs of `threads` threads and `smem` bytes of a kernel that the current device holds at once
+// CTAs of `threads` threads and `smem` bytes of a kernel that the device holds at once (its shared
+// memory limit is raised first)
 template <typename K>
-int resident_ctas(K kernel, int threads, size_t smem) {
+int resident_ctas(int dev, K kernel, int threads, size_t smem) {
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
-  int dev = 0, sms = 0, per = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  int sms = 0, per = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem) != cudaSuccess) return 0;
   return sms * per;
@@ -790,12 +790,12 @@ cudaError_t launch_plane_filter_batch(const BatchFilterInst<T>* inst, const CUte
   constexpr bool COMP = sizeof(T) == 4;
   const size_t smem = sizeof(T) * (kPlaneSlots * PlaneFilterBox<T>::FB +
                                    2 * (kPlaneWarps * kPlaneBatchRows + 8) * kPlaneCols);
-  static int resident = 0;
-  if (!resident) {
-    const int r = resident_ctas(k_plane_filter_batch<T, COMP, kPlaneBatchRows>, 32 * kPlaneWarps, smem);
-    if (r <= 0) return cudaErrorInvalidConfiguration;
-    resident = r;
-  }
+  static PerDevice held;
+  int dev = 0;
+  if (const cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return e;
+  const int resident = held.get(
+      dev, [&] { return resident_ctas(dev, k_plane_filter_batch<T, COMP, kPlaneBatchRows>, 32 * kPlaneWarps, smem); });
+  if (resident <= 0) return cudaErrorInvalidConfiguration;
   const int runs = std::max(1, resident / 4), per = (n + runs - 1) / runs;  // four fields
   k_plane_filter_batch<T, COMP, kPlaneBatchRows><<<dim3((n + per - 1) / per, 4), dim3(32, kPlaneWarps), smem, s>>>(
       inst, maps, tiles, n, per, p, err, wait_ns);

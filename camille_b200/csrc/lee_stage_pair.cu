@@ -178,12 +178,8 @@ template <int DIM, int TR>
 cudaError_t go_pair(const FieldMaps& z, const TmaStageParams<float>& p, int tiles, int chunks, cudaStream_t s) {
   constexpr int NS = DIM == 3 ? 2 * kFdHalf + 1 + StagePrefetch<float>::P : 1;
   const size_t sm = sizeof(float) * NS * (DIM + 2) * Box<float, kFdHalf>::FBP + NS * sizeof(uint64_t);
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_stage_pair<DIM, TR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static PerDevice smem;
+  if (const cudaError_t e = allow_smem(smem, k_stage_pair<DIM, TR>, sm); e != cudaSuccess) return e;
   k_stage_pair<DIM, TR><<<dim3(tiles, chunks), 128, sm, s>>>(z, p);
   return cudaGetLastError();
 }

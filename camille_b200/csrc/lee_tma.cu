@@ -585,14 +585,9 @@ size_t filter_smem() {
 
 template <typename T, int DIM, bool COMP, int TR>
 cudaError_t go_stage(const FieldMaps& z, const TmaStageParams<T>& p, int tiles, int chunks, cudaStream_t s) {
-  static bool attr = false;
+  static PerDevice smem;
   const size_t sm = stage_smem<T, DIM, COMP>();
-  if (!attr) {
-    cudaError_t e =
-        cudaFuncSetAttribute(k_stage_tma<T, DIM, COMP, TR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  if (const cudaError_t e = allow_smem(smem, k_stage_tma<T, DIM, COMP, TR>, sm); e != cudaSuccess) return e;
   k_stage_tma<T, DIM, COMP, TR><<<dim3(tiles, chunks), 256, sm, s>>>(z, p);
   return cudaGetLastError();
 }

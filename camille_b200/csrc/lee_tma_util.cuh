@@ -8,9 +8,26 @@
 #include <utility>
 
 #include <cuda.h>
+#include <cuda_runtime.h>
+
+#include "lee_per_device.h"
 
 namespace lee {
 namespace {
+
+// Raise a kernel's dynamic shared memory limit to `bytes` on the current device, which keeps it: once
+// per device and kernel (`done`).
+template <typename K>
+cudaError_t allow_smem(PerDevice& done, K kernel, size_t bytes) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  done.get(dev, [&] {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    return e == cudaSuccess ? 1 : 0;
+  });
+  return e;
+}
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
