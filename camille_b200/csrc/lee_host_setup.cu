@@ -545,9 +545,11 @@ int lee_prepare(lee_ctx* c) {
     // 2-D blocks: the direct kernels (lee_plane.cu), unless a kernel or form was asked for. Per
     // launch at 64 x 48 .. 640 x 640: FP32 stage 2.1 .. 6.0 us against 2.2 .. 7.4 (two-point TMA
     // kernel), FP64 2.7 .. 11.8 against 2.6 .. 12.7; on a 512 x 512 block with holes 7.9 against
-    // 10.2. A non-uniform mean without holes keeps the TMA kernels (384 x 96 FP32: 3.8 against 5.5)
-    b.plane_stage = dim == 2 && b.tma && c->stage_kernel < 0 && ((b.traits & kTrUniform) || b.has_holes);
-    b.plane_filter = dim == 2 && b.tma_filter && c->filter_kernel < 0 && c->filter_form == 0 && !c->increment_step &&
+    // 10.2. A non-uniform mean without holes keeps the TMA kernels (384 x 96 FP32: 3.8 against 5.5),
+    // and so do blocks of more rows than the direct kernels' grids hold
+    const bool plane = dim == 2 && b.ny <= kPlaneMaxRows;
+    b.plane_stage = plane && b.tma && c->stage_kernel < 0 && ((b.traits & kTrUniform) || b.has_holes);
+    b.plane_filter = plane && b.tma_filter && c->filter_kernel < 0 && c->filter_form == 0 && !c->increment_step &&
                      (c->hf == 2 || c->hf == 4 || c->hf == 5) && c->flt.nb <= kPlaneFilterNb;
     b.stage_chunk = b.filter_chunk = b.nz;
     if ((b.tma || b.tma_filter) && (rc = ensure_encoder(c))) return rc;

@@ -11,6 +11,7 @@ constexpr int kPlaneFdHalf = 2;    // the 4th-order difference
 constexpr int kPlaneFilterNb = 5;  // closure rows per line end, at most
 constexpr int kPlaneCols = 64;     // columns of a warp (two per thread)
 constexpr int kPlaneRows = 4;      // rows of a stage CTA (one per warp)
+constexpr int kPlaneMaxRows = 65535 * kPlaneRows;  // of a block: a grid's second dimension counts row groups
 constexpr int kPlaneBatchTall = 8; // rows of a batched stage tile
 constexpr int kPlaneSlots = 3;     // tiles whose boxes a batched filter CTA holds (the next ones in flight)
 constexpr int kPlaneWarps = 8;     // warps of a filter CTA

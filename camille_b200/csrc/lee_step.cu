@@ -293,7 +293,9 @@ cudaError_t launch_scalar_stage(const ScalarParams<T>& p, int comp, cudaStream_t
 
 template <typename T>
 cudaError_t launch_stage(const StageParams<T>& p, int comp, cudaStream_t s) {
-  if (p.fd.h == kWideHalf && !p.code[0]) {  // (lines have at least 2 h + 1 points, checked at setup)
+  // (lines have at least 2 h + 1 points, checked at setup; the grid's second dimension counts groups
+  // of four rows, k_stage's of eight)
+  if (p.fd.h == kWideHalf && !p.code[0] && p.ny <= 65535 * 4) {
     if (p.dim == 2) return comp ? go_wide<T, 2, true>(p, s) : go_wide<T, 2, false>(p, s);
     return comp ? go_wide<T, 3, true>(p, s) : go_wide<T, 3, false>(p, s);
   }
