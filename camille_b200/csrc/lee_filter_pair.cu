@@ -62,9 +62,9 @@ struct Own<float> {
   using W = float2;
   static constexpr int N = 2;
   static __device__ __forceinline__ W zero() { return make_float2(0.f, 0.f); }
-  // (1 - b) x + b f
+  // (1 - b) x + b f with the roundings of the other forms (lee_tma.cu)
   static __device__ __forceinline__ W blend(float b, W x, W f) {
-    return make_float2((1.f - b) * x.x + b * f.x, (1.f - b) * x.y + b * f.y);
+    return make_float2(fmaf(b, f.x, (1.f - b) * x.x), fmaf(b, f.y, (1.f - b) * x.y));
   }
 };
 template <>
@@ -72,7 +72,7 @@ struct Own<double> {
   using W = double;
   static constexpr int N = 1;
   static __device__ __forceinline__ W zero() { return 0.0; }
-  static __device__ __forceinline__ W blend(double b, W x, W f) { return (1.0 - b) * x + b * f; }
+  static __device__ __forceinline__ W blend(double b, W x, W f) { return fma(b, f, (1.0 - b) * x); }
 };
 template <typename T>
 __device__ __forceinline__ typename Own<T>::W ld2(const T* p) {

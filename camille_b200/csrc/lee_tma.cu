@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(256) k_filter_tma_row(const __grid_constant__ 
     const long long l = lf;
     const bool hole = HOLES && P.iblank[l] == 1;  // temporal::iblank_correction
     if (!COMP) {
-      P.out[v][l] = hole ? T(0) : (T(1) - P.blend) * x0 + P.blend * fz;
+      P.out[v][l] = hole ? T(0) : fma_t(P.blend, fz, (T(1) - P.blend) * x0);
     } else {
       const T D = DIM == 3 ? dsum + fz : dsum;
       const T t = P.blend * D + e0;
@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(256) k_filter_tma(const __grid_constant__ Fiel
       }
       const long long l = i + (long long)P.px * (jr[r] + (long long)P.ny * k);
       if (!COMP) {
-        P.out[v][l] = (T(1) - P.blend) * x0 + P.blend * fz;
+        P.out[v][l] = fma_t(P.blend, fz, (T(1) - P.blend) * x0);
       } else {
         const T D = DIM == 3 ? dsum + fz : dsum;
         const T t = P.blend * D + ef[r];
