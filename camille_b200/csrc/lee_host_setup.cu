@@ -149,8 +149,9 @@ int build_mean(lee_ctx* c, BlockData& b) {
   Coef<T> k[20];
   mean_coefs<T>(b, k);
   b.mean_terms = 0;
-  for (int q = 0; q < 3; ++q) b.mean_terms |= (k[kMeanGs + q].zero ? 0 : 1) | (k[kMeanGp + q].zero ? 0 : 4);
-  for (int q = 0; q < 9; ++q) b.mean_terms |= k[kMeanGu + q].zero ? 0 : 2;
+  for (int q = 0; q < 3; ++q)
+    b.mean_terms |= (k[kMeanGs + q].zero ? 0 : kMeanHasGs | mean_gs(q)) | (k[kMeanGp + q].zero ? 0 : kMeanHasGp | mean_gp(q));
+  for (int q = 0; q < 9; ++q) b.mean_terms |= k[kMeanGu + q].zero ? 0 : kMeanHasGu | mean_gu(q / 3, q % 3);
   T h[2 * 21];
   for (int q = 0; q < 20; ++q) h[2 * q] = h[2 * q + 1] = k[q].zero ? T(0) : k[q].c;
   h[2 * kMeanIpb] = h[2 * kMeanIpb + 1] = T(1) / k[kMeanPb].c;

@@ -153,8 +153,14 @@ struct StageParams {
   // pair of points reads it as one), so that the kernels load them all without a branch
   const T* mean[21];
   int mean_mask[21];
-  int mean_terms;  // which gradients are not identically zero: bit 0 s_bar, 1 u_bar, 2 p_bar
+  // which mean gradients are not identically zero: some component of a field's
+  // (kMeanHas*), and each component's own bit (mean_gs, mean_gp, mean_gu)
+  int mean_terms;
 };
+__host__ __device__ constexpr int mean_gs(int x) { return 8 << x; }                    // d s_bar/dx_x
+__host__ __device__ constexpr int mean_gp(int x) { return 64 << x; }                   // d p_bar/dx_x
+__host__ __device__ constexpr int mean_gu(int a, int x) { return 512 << (a * 3 + x); }  // d u_bar_a/dx_x
+constexpr int kMeanHasGs = 1, kMeanHasGu = 2, kMeanHasGp = 4;  // bits of StageParams::mean_terms
 constexpr int kMeanUb = 0, kMeanRbi = 3, kMeanPb = 4, kMeanGs = 5, kMeanGu = 8, kMeanGp = 17, kMeanIpb = 20;
 
 template <typename T>

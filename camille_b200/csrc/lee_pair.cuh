@@ -62,12 +62,12 @@ __device__ __forceinline__ void gather_mean_pair(const StageParams<float>& p, un
   m.pb = at(kMeanPb);
 #pragma unroll
   for (int x = 0; x < DIM; ++x) {
-    m.gs[x] = (p.mean_terms & 1) ? at(kMeanGs + x) : f2(0.f);
-    m.gp[x] = (p.mean_terms & 4) ? at(kMeanGp + x) : f2(0.f);
+    m.gs[x] = (p.mean_terms & kMeanHasGs) ? at(kMeanGs + x) : f2(0.f);
+    m.gp[x] = (p.mean_terms & kMeanHasGp) ? at(kMeanGp + x) : f2(0.f);
 #pragma unroll
-    for (int a = 0; a < DIM; ++a) m.gu[a][x] = (p.mean_terms & 2) ? at(kMeanGu + a * 3 + x) : f2(0.f);
+    for (int a = 0; a < DIM; ++a) m.gu[a][x] = (p.mean_terms & kMeanHasGu) ? at(kMeanGu + a * 3 + x) : f2(0.f);
   }
-  m.rr = !(p.mean_terms & 2) ? f2(0.f) : (reads_rho_prev<float, TR>(p) ? ld2(p.rho_prev + l) : at(kMeanIpb));
+  m.rr = !(p.mean_terms & kMeanHasGu) ? f2(0.f) : (reads_rho_prev<float, TR>(p) ? ld2(p.rho_prev + l) : at(kMeanIpb));
 }
 
 // rhs_mean_terms (lee_point.cuh) of a pair
@@ -83,7 +83,7 @@ __device__ __forceinline__ void pair_mean_terms(const StageParams<float>& p, con
     nu[x] = mul(q[1 + x], neg);
   }
   F2 rr = f2(0.f);
-  if (p.mean_terms & 2) {
+  if (p.mean_terms & kMeanHasGu) {
     rr = m.rr;
     if (!reads_rho_prev<float, TR>(p)) rr = fma2(mul(q[P], f2(p.inv_gamma)), m.rr, mul(q[0], neg));
   }
@@ -92,7 +92,7 @@ __device__ __forceinline__ void pair_mean_terms(const StageParams<float>& p, con
 #pragma unroll
     for (int x = 0; x < DIM; ++x) {
       if (x) t = fma2(nub[x], g[0][x], t);
-      if (p.mean_terms & 1) t = fma2(nu[x], m.gs[x], t);
+      if (p.mean_terms & kMeanHasGs) t = fma2(nu[x], m.gs[x], t);
     }
     r[0] = t;
   }
@@ -103,7 +103,7 @@ __device__ __forceinline__ void pair_mean_terms(const StageParams<float>& p, con
 #pragma unroll
     for (int x = 0; x < DIM; ++x) {
       if (x) t = fma2(nub[x], g[1 + a][x], t);
-      if (p.mean_terms & 2) t = fma2(fma2(rr, nub[x], nu[x]), m.gu[a][x], t);
+      if (p.mean_terms & kMeanHasGu) t = fma2(fma2(rr, nub[x], nu[x]), m.gu[a][x], t);
     }
     r[1 + a] = fma2(mul(g[P][a], neg), m.rbi, t);
   }
@@ -112,9 +112,9 @@ __device__ __forceinline__ void pair_mean_terms(const StageParams<float>& p, con
 #pragma unroll
     for (int x = 0; x < DIM; ++x) {
       if (x) t = fma2(nub[x], g[P][x], t);
-      if (p.mean_terms & 4) t = fma2(nu[x], m.gp[x], t);
+      if (p.mean_terms & kMeanHasGp) t = fma2(nu[x], m.gp[x], t);
       t = fma2(ngpb, g[1 + x][x], t);
-      if (p.mean_terms & 2) t = fma2(ngq, m.gu[x][x], t);
+      if (p.mean_terms & kMeanHasGu) t = fma2(ngq, m.gu[x][x], t);
     }
     r[P] = t;
   }

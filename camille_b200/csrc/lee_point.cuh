@@ -73,38 +73,69 @@ __device__ __forceinline__ void gather(const StageParams<T>& p, I l, PointIn<T, 
   in.sg = (TR & kTrSponge) ? __ldg(p.sigma + l) : T(0);
 }
 
-// The mean flow at a point of a non-uniform block.
-template <typename T, int DIM>
-struct PointMean {
-  T ub[DIM], rbi, pb, gs[DIM], gu[DIM][DIM], gp[DIM];
-  T rr;  // rho'/rho_bar of the previous step (stages that read it), else 1 / p_bar
-};
-
 template <typename T, int TR>
 __device__ __forceinline__ bool reads_rho_prev(const StageParams<T>& p) {
   return (Kind<TR>::first(p) || Kind<TR>::rhs(p)) && p.rho_prev;
 }
 
+// The mean flow at a point of a non-uniform block, in one of two forms with the same values: read
+// into registers ahead, every component of a gradient that is not identically zero (PointMean, where
+// registers are to spare: the 11-point and direct 2-D kernels, the pairs of lee_pair.cuh), or read
+// where it is used, component by component (MeanAt: k_stage and k_stage_tma, whose registers are
+// full). k_stage_tma, 96^3, per launch: FP64 with one gradient component 80 us, read ahead 105; with
+// all fifteen 130 and 129. FP32 51 and 67, 81 and 90. k_stage, FP32, 65^3 with two components: 56 and
+// 76. The 11-point kernel, FP32: read ahead 78 and 85, where used 83 and 109.
+template <typename T, int DIM>
+struct PointMean {
+  T ub_[DIM], rbi_, pb_, gs_[DIM], gu_[DIM][DIM], gp_[DIM];
+  T rr_;  // rho'/rho_bar of the previous step (stages that read it), else 1 / p_bar
+  __device__ __forceinline__ T ub(int x) const { return ub_[x]; }
+  __device__ __forceinline__ T rbi() const { return rbi_; }
+  __device__ __forceinline__ T pb() const { return pb_; }
+  __device__ __forceinline__ T gs(int x) const { return gs_[x]; }
+  __device__ __forceinline__ T gp(int x) const { return gp_[x]; }
+  __device__ __forceinline__ T gu(int a, int x) const { return gu_[a][x]; }
+  __device__ __forceinline__ T rho_prev() const { return rr_; }
+  __device__ __forceinline__ T ipb() const { return rr_; }
+  static __device__ __forceinline__ bool has(int terms, int field, int) { return (terms & field) != 0; }
+};
+
 template <typename T, int DIM, int TR, typename I>
 __device__ __forceinline__ void gather_mean(const StageParams<T>& p, I l, PointMean<T, DIM>& m) {
   auto at = [&](int k) { return __ldg(p.mean[k] + (l & (I)p.mean_mask[k])); };
 #pragma unroll
-  for (int x = 0; x < DIM; ++x) m.ub[x] = at(kMeanUb + x);
-  m.rbi = at(kMeanRbi);
-  m.pb = at(kMeanPb);
+  for (int x = 0; x < DIM; ++x) m.ub_[x] = at(kMeanUb + x);
+  m.rbi_ = at(kMeanRbi);
+  m.pb_ = at(kMeanPb);
 #pragma unroll
   for (int x = 0; x < DIM; ++x) {
-    m.gs[x] = (p.mean_terms & 1) ? at(kMeanGs + x) : T(0);
-    m.gp[x] = (p.mean_terms & 4) ? at(kMeanGp + x) : T(0);
+    m.gs_[x] = (p.mean_terms & kMeanHasGs) ? at(kMeanGs + x) : T(0);
+    m.gp_[x] = (p.mean_terms & kMeanHasGp) ? at(kMeanGp + x) : T(0);
 #pragma unroll
-    for (int a = 0; a < DIM; ++a) m.gu[a][x] = (p.mean_terms & 2) ? at(kMeanGu + a * 3 + x) : T(0);
+    for (int a = 0; a < DIM; ++a) m.gu_[a][x] = (p.mean_terms & kMeanHasGu) ? at(kMeanGu + a * 3 + x) : T(0);
   }
-  m.rr = !(p.mean_terms & 2) ? T(0) : (reads_rho_prev<T, TR>(p) ? p.rho_prev[l] : at(kMeanIpb));
+  m.rr_ = !(p.mean_terms & kMeanHasGu) ? T(0) : (reads_rho_prev<T, TR>(p) ? p.rho_prev[l] : at(kMeanIpb));
 }
 
-template <typename T, int DIM, int TR>
+template <typename T, typename I>
+struct MeanAt {
+  const StageParams<T>& p;
+  I l;
+  __device__ __forceinline__ T at(int k) const { return __ldg(p.mean[k] + (l & (I)p.mean_mask[k])); }
+  __device__ __forceinline__ T ub(int x) const { return at(kMeanUb + x); }
+  __device__ __forceinline__ T rbi() const { return at(kMeanRbi); }
+  __device__ __forceinline__ T pb() const { return at(kMeanPb); }
+  __device__ __forceinline__ T gs(int x) const { return at(kMeanGs + x); }
+  __device__ __forceinline__ T gp(int x) const { return at(kMeanGp + x); }
+  __device__ __forceinline__ T gu(int a, int x) const { return at(kMeanGu + a * 3 + x); }
+  __device__ __forceinline__ T rho_prev() const { return p.rho_prev[l]; }
+  __device__ __forceinline__ T ipb() const { return at(kMeanIpb); }
+  static __device__ __forceinline__ bool has(int terms, int, int component) { return (terms & component) != 0; }
+};
+
+template <typename T, int DIM, int TR, typename M>
 __device__ __forceinline__ void rhs_mean_terms(const StageParams<T>& p, const T (&g)[DIM + 2][DIM],
-                                               const T (&q)[DIM + 2], const PointMean<T, DIM>& m, T (&r)[DIM + 2]);
+                                               const T (&q)[DIM + 2], const M& m, T (&r)[DIM + 2]);
 template <typename T, int DIM, bool COMP, int TR, typename I>
 __device__ __forceinline__ void rk_update(const StageParams<T>& p, I l, const T (&q)[DIM + 2],
                                           const PointIn<T, DIM>& in, const T (&r)[DIM + 2]);
@@ -112,11 +143,10 @@ __device__ __forceinline__ void rk_update(const StageParams<T>& p, I l, const T 
 // D[v][d]: computational-space derivative of field v along direction d; q[v]: the
 // stage input at the point; in: the gathered inputs, mean: the mean flow of a non-uniform block.
 // r receives the right-hand side.
-template <typename T, int DIM, int TR, typename I>
+template <typename T, int DIM, int TR, typename I, typename M>
 __device__ __forceinline__ void rhs_point(const StageParams<T>& p, I l, int i, int j, int k,
                                           const T (&D)[DIM + 2][DIM], const T (&q)[DIM + 2],
-                                          const PointIn<T, DIM>& in, const PointMean<T, DIM>& mean,
-                                          T (&r)[DIM + 2]) {
+                                          const PointIn<T, DIM>& in, const M& mean, T (&r)[DIM + 2]) {
   constexpr int V = DIM + 2;
   constexpr int P = DIM + 1;
   // physical gradients g[v][x] = sum_d JM[d][x] D_d f_v (take_derivative_xyz, :1802-1826)
@@ -132,10 +162,10 @@ __device__ __forceinline__ void rhs_point(const StageParams<T>& p, I l, int i, i
     }
   }
   constexpr bool UNI = (TR & kTrUniform) != 0;
-  T ub[DIM];
-#pragma unroll
-  for (int x = 0; x < DIM; ++x) ub[x] = UNI ? p.ubar[x].c : mean.ub[x];
   if (UNI) {
+    T ub[DIM];
+#pragma unroll
+    for (int x = 0; x < DIM; ++x) ub[x] = p.ubar[x].c;
     // uniform mean flow: every mean-gradient term vanishes
     T rs = T(0);
 #pragma unroll
@@ -203,51 +233,55 @@ __device__ __forceinline__ void rhs_point(const StageParams<T>& p, I l, int i, i
 
 // The right-hand side at a point, then the stage update: writes the next stage input and the
 // accumulator.
-template <typename T, int DIM, bool COMP, int TR, typename I>
+template <typename T, int DIM, bool COMP, int TR, typename I, typename M>
 __device__ __forceinline__ void rhs_update(const StageParams<T>& p, I l, int i, int j, int k,
                                            const T (&D)[DIM + 2][DIM], const T (&q)[DIM + 2],
-                                           const PointIn<T, DIM>& in, const PointMean<T, DIM>& mean) {
+                                           const PointIn<T, DIM>& in, const M& mean) {
   T r[DIM + 2];
   rhs_point<T, DIM, TR>(p, l, i, j, k, D, q, in, mean, r);
   rk_update<T, DIM, COMP, TR>(p, l, q, in, r);
 }
 
 // The LEE right-hand side of a non-uniform mean flow; gradients that are identically zero are
-// skipped by the field they belong to.
-template <typename T, int DIM, int TR>
+// skipped, by the field or component that M tells apart.
+template <typename T, int DIM, int TR, typename M>
 __device__ __forceinline__ void rhs_mean_terms(const StageParams<T>& p, const T (&g)[DIM + 2][DIM],
-                                               const T (&q)[DIM + 2], const PointMean<T, DIM>& m, T (&r)[DIM + 2]) {
+                                               const T (&q)[DIM + 2], const M& m, T (&r)[DIM + 2]) {
   constexpr int P = DIM + 1;
+  const int has = p.mean_terms;
+  T ub[DIM];
+#pragma unroll
+  for (int x = 0; x < DIM; ++x) ub[x] = m.ub(x);
   {
     T rs = T(0);
 #pragma unroll
     for (int x = 0; x < DIM; ++x) {
-      rs = fma_t(-m.ub[x], g[0][x], rs);
-      if (p.mean_terms & 1) rs = fma_t(-q[1 + x], m.gs[x], rs);
+      rs = fma_t(-ub[x], g[0][x], rs);
+      if (M::has(has, kMeanHasGs, mean_gs(x))) rs = fma_t(-q[1 + x], m.gs(x), rs);
     }
     r[0] = rs;
   }
   T rr = T(0);
-  if (p.mean_terms & 2) rr = reads_rho_prev<T, TR>(p) ? m.rr : fma_t(q[P] * p.inv_gamma, m.rr, -q[0]);
+  if (has & kMeanHasGu) rr = reads_rho_prev<T, TR>(p) ? m.rho_prev() : fma_t(q[P] * p.inv_gamma, m.ipb(), -q[0]);
 #pragma unroll
   for (int a = 0; a < DIM; ++a) {
     T ru = T(0);
 #pragma unroll
     for (int x = 0; x < DIM; ++x) {
-      ru = fma_t(-m.ub[x], g[1 + a][x], ru);
-      if (p.mean_terms & 2) ru = fma_t(-fma_t(rr, m.ub[x], q[1 + x]), m.gu[a][x], ru);
+      ru = fma_t(-ub[x], g[1 + a][x], ru);
+      if (M::has(has, kMeanHasGu, mean_gu(a, x))) ru = fma_t(-fma_t(rr, ub[x], q[1 + x]), m.gu(a, x), ru);
     }
-    r[1 + a] = fma_t(-g[P][a], m.rbi, ru);
+    r[1 + a] = fma_t(-g[P][a], m.rbi(), ru);
   }
   {
     T rp = T(0);
-    const T gpb = p.gamma * m.pb, gq = p.gamma * q[P];
+    const T gpb = p.gamma * m.pb(), gq = p.gamma * q[P];
 #pragma unroll
     for (int x = 0; x < DIM; ++x) {
-      rp = fma_t(-m.ub[x], g[P][x], rp);
-      if (p.mean_terms & 4) rp = fma_t(-q[1 + x], m.gp[x], rp);
+      rp = fma_t(-ub[x], g[P][x], rp);
+      if (M::has(has, kMeanHasGp, mean_gp(x))) rp = fma_t(-q[1 + x], m.gp(x), rp);
       rp = fma_t(-gpb, g[1 + x][x], rp);
-      if (p.mean_terms & 2) rp = fma_t(-gq, m.gu[x][x], rp);
+      if (M::has(has, kMeanHasGu, mean_gu(x, x))) rp = fma_t(-gq, m.gu(x, x), rp);
     }
     r[P] = rp;
   }

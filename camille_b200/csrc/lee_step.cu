@@ -65,8 +65,6 @@ __global__ void __launch_bounds__(256) k_stage(StageParams<T> p) {
   const long long sd[3] = {1, p.px, nxy};
   PointIn<T, DIM> in;
   gather<T, DIM, COMP, kTrGeneric>(p, l, in);
-  PointMean<T, DIM> mean;
-  gather_mean<T, DIM, kTrGeneric>(p, l, mean);
   T D[V][DIM], q[V];
 #pragma unroll
   for (int v = 0; v < V; ++v) {
@@ -74,7 +72,7 @@ __global__ void __launch_bounds__(256) k_stage(StageParams<T> p) {
     for (int d = 0; d < DIM; ++d) D[v][d] = dop<T>(p.fd, p.zin[v], l, pos[d], nn[d], sd[d], p.code[d]);
     q[v] = p.zin[v][l];
   }
-  rhs_update<T, DIM, COMP, kTrGeneric>(p, l, i, j, k, D, q, in, mean);
+  rhs_update<T, DIM, COMP, kTrGeneric>(p, l, i, j, k, D, q, in, MeanAt<T, long long>{p, l});
 }
 
 // k_stage for the 11-point difference on a block without closure codes: the half-width is known at

@@ -98,8 +98,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2)
     const unsigned lk = lij + nxy * (unsigned)k;
     if (PIPE && active && k + 1 < k1) gather<T, DIM, COMP, TR>(s, lk + nxy, nxt);
     if (!PIPE && active) gather<T, DIM, COMP, TR>(s, lk, cur);
-    PointMean<T, DIM> mean;  // (in flight during the wait)
-    if (!(TR & kTrUniform) && active) gather_mean<T, DIM, TR>(s, lk, mean);
     bool failed = false;
     const int need = DIM == 3 ? min(phi, k + H) : 0;
     // `waited` stays at a plane whose wait gave up, so the drain below starts there
@@ -168,7 +166,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2)
           D[v][DIM - 1] = dz;
         }
       }
-      rhs_update<T, DIM, COMP, TR>(s, lk, i, j, k, D, q, cur, mean);
+      rhs_update<T, DIM, COMP, TR>(s, lk, i, j, k, D, q, cur, MeanAt<T, unsigned>{s, lk});
     }
     sk = sk + 1 == NS ? 0 : sk + 1;
     return true;
