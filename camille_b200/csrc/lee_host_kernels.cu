@@ -312,6 +312,10 @@ int autotune(lee_ctx* c, BlockData& b) {
   // length, so that CTA counts that fill whole waves of the GPU are among the candidates)
   std::vector<int> ladder = {8, 16, 24, 32, 48, 64, 96, 128, 192, 256};
   if (b.nz < ladder[0]) ladder.push_back(b.nz);
+  // launches of a small block last about 10 us, in the order of what an event resolves: several
+  // between two events
+  const bool small = b.N < (1 << 19);
+  const int launches = small ? 6 : 2;
   std::vector<int> splits;
   for (int q = 1; q <= 24; ++q) {
     const int ch = (b.nz + q - 1) / q;
@@ -335,19 +339,22 @@ int autotune(lee_ctx* c, BlockData& b) {
     float best = 1e30f;
     int best_chunk = b.nz, best_kind = which == 0 ? b.stage_px : b.filter_px, best_ry = b.filter_ry;
     bool best_pair = b.filter_pair;
-    // the best scalar form (one or two rows) and its chunk, kept for the transposed filter of
-    // the adjoint, which the two-point kernel does not run
+    // the best scalar form (one or two rows) and its chunk, kept for the adjoint's transposed filter
+    // where form 3 does not run
     float best_scalar = 1e30f;
     int best_scalar_chunk = b.nz, best_scalar_ry = b.filter_ry;
-    // the scalar filter's forms (1: one tile row per thread row, 2: two rows, 3: two points per
-    // thread) are timed with the chunk: each point's arithmetic is the same in all three
+    // the scalar filter's forms (1: one tile row per thread row, 2: two rows, 3: lee_filter_pair.cu)
+    // are timed with the chunk: each point's arithmetic is the same in all three. Form 3 is the
+    // fastest on large blocks (FP32 0.35 against 0.61 ms at 256^3, FP64 0.13 against 0.19 at 160 x 144
+    // x 128); below about 40^3 its 64 x 16 tiles are too few (20^3 FP32 14.8 us against 12.7)
     const int nry = which == 1 && b.filter_form == 0 ? 3 : 1;
     // the ladder for every form, then the filter's other splits for the form that won there (a
-    // third of the launches of every split for every form: 12 instead of 40 ms at 129 x 113 x 97)
+    // third of the launches of every split for every form: 12 instead of 40 ms at 129 x 113 x 97);
+    // on a small block, where the best chunks are shorter than the ladder's, every split for every form
     int best_kq = 0;
     for (int phase = 0; phase < (d3 && which == 1 ? 2 : 1); ++phase) {
       for (int kq = 0; kq < (which == 1 ? nkinds : nskinds) * nry; ++kq) {
-        if (phase == 1 && kq != best_kq) continue;
+        if (phase == 1 && kq != best_kq && !small) continue;
         if (which == 0) {
           b.stage_px = skinds[kq];
         } else {
@@ -358,18 +365,15 @@ int autotune(lee_ctx* c, BlockData& b) {
           if (b.filter_form == 0 && (b.filter_px > 0 || b.has_holes || (c->comp && c->increment_step)) && form > 1)
             continue;
           if (form == 3 && !b.filter_pair_ok) continue;
-          // (where it applies, form 3, two rows per thread, is the fastest: FP32 0.35 against 0.61 ms
-          // at 256^3, FP64 0.13 against 0.19 at 160 x 144 x 128)
-          if (b.filter_form == 0 && b.filter_pair_ok && form != 3 && !(c->comp && c->increment_step)) continue;
           b.filter_ry = form == 2 ? 2 : 1;
           b.filter_pair = form == 3;
           set_filter_tiles(c, b);
         }
         for (int ch : (d3 ? (phase == 1 ? splits : ladder) : cands2)) {
           if (d3 && ch > b.nz) continue;
-          float tsum = 0.f;
-          for (int rep = 0; rep < 3; ++rep) {  // the first run warms up
-            CK(cudaEventRecord(e0, c->stream));
+          float ms = 0.f;
+          for (int rep = 0; rep <= launches; ++rep) {  // the first run warms up
+            if (rep == 1) CK(cudaEventRecord(e0, c->stream));
             int rc;
             if (which == 0) {
               StageParams<T> p;
@@ -393,19 +397,17 @@ int autotune(lee_ctx* c, BlockData& b) {
                            : launch_filter_fused<T>(c, b, b.acc, nullptr, b.zb[0], nullptr, chunk);
             }
             if (rc) return rc;
-            CK(cudaEventRecord(e1, c->stream));
-            CK(cudaEventSynchronize(e1));
-            float ms = 0.f;
-            CK(cudaEventElapsedTime(&ms, e0, e1));
-            if (rep > 0) tsum += ms;
           }
-          if (which == 1 && !b.filter_pair && tsum < best_scalar) {
-            best_scalar = tsum;
+          CK(cudaEventRecord(e1, c->stream));
+          CK(cudaEventSynchronize(e1));
+          CK(cudaEventElapsedTime(&ms, e0, e1));
+          if (which == 1 && !b.filter_pair && ms < best_scalar) {
+            best_scalar = ms;
             best_scalar_chunk = d3 ? ch : b.nz;
             best_scalar_ry = b.filter_ry;
           }
-          if (tsum < best) {
-            best = tsum;
+          if (ms < best) {
+            best = ms;
             best_kq = kq;
             best_chunk = d3 ? ch : b.nz;
             best_kind = which == 0 ? b.stage_px : b.filter_px;
