@@ -209,6 +209,7 @@ int lee_create(const lee_config* cfg, lee_ctx** out) {
   c->wst_ok = c->fd.h == kFdHalf && class_weights(c->fd, kFdHalf, &c->wst[0][0], 5);
   c->blk.resize((size_t)cfg->num_blocks);
   e = cudaSetDevice(cfg->device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, cfg->device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_err, 2 * sizeof(int));
   if (e == cudaSuccess) e = cudaMemsetAsync(c->d_err, 0, 2 * sizeof(int), c->stream);

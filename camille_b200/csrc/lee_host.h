@@ -160,6 +160,7 @@ struct StepGraph {
 struct lee_ctx {
   lee_config cfg;
   int V = 0;
+  int sms = 148;  // multiprocessors of the device
   size_t esz = 8;
   bool comp = false;
   OpTable fd{}, flt{}, fltd{};
@@ -379,7 +380,9 @@ int filter_box(const lee_ctx* c, int h, int form, int* bx, int* by);
 int filter_tiles(const BlockData& b);
 int filter_tiles_form(const BlockData& b, int ry);  // the scalar fused filter's tiles in form ry (1 or 2)
 void set_filter_tiles(const lee_ctx* c, BlockData& b);
-int plane_filter_rows(const BlockData& b, int V);
+bool plane_stage_pays(const lee_ctx* c, const BlockData& b);
+bool plane_filter_pays(const lee_ctx* c, const BlockData& b);
+int plane_filter_rows(const lee_ctx* c, const BlockData& b);
 template <typename T>
 void plane_filter_common(const lee_ctx* c, PlaneFilter<T>& p);
 template <typename T>

@@ -200,8 +200,7 @@ int batch_setup(lee_ctx* c) {
   CK(cudaMalloc(&d_fs, fs.size() * sizeof(fs[0])));
   CK(cudaMemcpyAsync(d_pr, pr.data(), pr.size() * sizeof(pr[0]), cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(d_fs, fs.data(), fs.size() * sizeof(fs[0]), cudaMemcpyHostToDevice, c->stream));
-  int nsm = 148;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->cfg.device);
+  const int nsm = c->sms;
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
@@ -370,8 +369,7 @@ int lee_set_batch_shapes(lee_ctx* c, int stage_shape, int filter_shape) {
     return fail(c, LEE_ERR_ARG, "shape index");
   CK(cudaSetDevice(c->cfg.device));
   auto& bt = c->batch;
-  int nsm = 148;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->cfg.device);
+  const int nsm = c->sms;
   const std::vector<int4> ts = batch_tiles(c, stage_shape), tf = batch_tiles(c, filter_shape);
   int rc;
   if ((rc = dalloc(c, &bt.d_stiles, ts.size())) || (rc = dalloc(c, &bt.d_ftiles, tf.size()))) return rc;

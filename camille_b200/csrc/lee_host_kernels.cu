@@ -194,12 +194,45 @@ int launch_stage_any(lee_ctx* c, BlockData& b, const StageParams<T>& p, void* co
   return LEE_OK;
 }
 
+// CTAs of a direct 2-D filter launch of two rows per warp.
+static long long plane_filter_ctas(const lee_ctx* c, const BlockData& b) {
+  return (long long)((b.nx + kPlaneCols - 1) / kPlaneCols) * ((b.ny + 2 * kPlaneWarps - 1) / (2 * kPlaneWarps)) * c->V;
+}
+
 // Rows a warp of the direct 2-D filter finishes: two filter 1.5 rows along xi per row finished
 // instead of 2, one gives twice the CTAs. Per launch at 64 x 48 .. 640 x 640 FP32 2.4 .. 8.8 us
 // against 2.4 .. 13.0 (the TMA forms), FP64 2.5 .. 13.0 against 2.6 .. 15.9.
-int plane_filter_rows(const BlockData& b, int V) {
-  const long long ctas = (long long)((b.nx + kPlaneCols - 1) / kPlaneCols) * ((b.ny + 2 * kPlaneWarps - 1) / (2 * kPlaneWarps)) * V;
-  return ctas >= 148 * 2 ? 2 : 1;
+int plane_filter_rows(const lee_ctx* c, const BlockData& b) { return plane_filter_ctas(c, b) >= c->sms * 2 ? 2 : 1; }
+
+// Whether the direct stage kernel serves a 2-D block better than the TMA kernels it has the bits of.
+// Its tiles are 64 columns wide, theirs 32: once the launch holds more CTAs than the GPU does, idle
+// columns cost. FP64 us per step, direct and TMA stages (the two-column rule: half of the tile idle):
+// 12 x 512 14.6 and 16.6, 12 x 1000 20.6 and 18.6, 12 x 4000 47.7 and 35.3; (a quarter idle) 72 x 512
+// 18.7 and 18.7, 72 x 1200 31.6 and 30.5, 72 x 4000 75.9 and 65.7; (a sixth) 160 x 600 26.8 and 26.8,
+// 160 x 4000 121 and 112; (a tenth) 264 x 4000 201 and 200; 513 x 4000 360 and 367. Full tiles, one
+// column of them: 64 x 1600 29.0 and 28.8, 64 x 8192 91 and 87; more: 400 x 4000 279 and 283. FP32
+// loses to them where half of the tile is idle alone: 12 x 2400 20.7 and 20.6, 12 x 4000 26.8 and 24.7,
+// 32 x 8192 45 and 41, 36 x 8192 47 and 55. Around holes the TMA kernels run one point per thread:
+// FP64 36 x 8192 88 and 109, 72 x 8192 183 and 172 (with their filter 200).
+bool plane_stage_pays(const lee_ctx* c, const BlockData& b) {
+  const long long wide = (b.nx + kPlaneCols - 1) / kPlaneCols, narrow = (b.nx + kTileX - 1) / kTileX;
+  const long long ctas = wide * ((b.ny + kPlaneRows - 1) / kPlaneRows);
+  const long long idle2 = ctas * (2 * wide - narrow) / wide;  // half tiles with no columns
+  if (b.nx <= kTileX) return ctas <= (c->comp ? 4 : 1) * c->sms;
+  if (c->comp || b.has_holes) return true;
+  if (b.nx <= kPlaneCols) return ctas <= 6 * c->sms;
+  return idle2 < c->sms || 16 * wide < 9 * narrow;
+}
+
+// Whether the direct filter does (FP32: it does). FP64, the 11-point filter, whose halo of ten rows
+// is filtered again by every 16 rows: us per step, direct and TMA, 256 x 256 20.6 and 20.6, 512 x 512
+// 47.7 and 47.1, 1000 x 1000 193 and 183, 12 x 1500 24.7 and 22.7. The other widths where half of the
+// tile is idle: 8th order 32 x 2500 28.8 and 28.8, 32 x 4000 37.0 and 35.0; 96 x 6000 102 and 102.
+bool plane_filter_pays(const lee_ctx* c, const BlockData& b) {
+  if (c->comp || b.has_holes) return true;
+  const long long ctas = plane_filter_ctas(c, b);
+  if (c->hf == 5) return 2 * ctas <= 5 * c->sms;
+  return b.nx > kTileX || ctas <= 6 * c->sms;
 }
 
 template <typename T>
@@ -221,7 +254,7 @@ int launch_filter_fused(lee_ctx* c, BlockData& b, void* const* in, void* const* 
     pf.nx = b.nx;
     pf.ny = b.ny;
     pf.px = b.px;
-    pf.rows = plane_filter_rows(b, c->V);
+    pf.rows = plane_filter_rows(c, b);
     pf.overlap = c->blk.size() == 1 && !c->timing;
     if (b.has_holes) {
       pf.code[0] = b.d_tcode_flt[0];

@@ -549,9 +549,10 @@ int lee_prepare(lee_ctx* c) {
     // 10.2. A non-uniform mean without holes keeps the TMA kernels (384 x 96 FP32: 3.8 against 5.5),
     // and so do blocks of more rows than the direct kernels' grids hold
     const bool plane = dim == 2 && b.ny <= kPlaneMaxRows;
-    b.plane_stage = plane && b.tma && c->stage_kernel < 0 && ((b.traits & kTrUniform) || b.has_holes);
+    b.plane_stage = plane && b.tma && c->stage_kernel < 0 && ((b.traits & kTrUniform) || b.has_holes) &&
+                    plane_stage_pays(c, b);
     b.plane_filter = plane && b.tma_filter && c->filter_kernel < 0 && c->filter_form == 0 && !c->increment_step &&
-                     (c->hf == 2 || c->hf == 4 || c->hf == 5) && c->flt.nb <= kPlaneFilterNb;
+                     (c->hf == 2 || c->hf == 4 || c->hf == 5) && c->flt.nb <= kPlaneFilterNb && plane_filter_pays(c, b);
     b.stage_chunk = b.filter_chunk = b.nz;
     if ((b.tma || b.tma_filter) && (rc = ensure_encoder(c))) return rc;
     if ((rc = c->comp ? autotune<float>(c, b) : autotune<double>(c, b))) return rc;
