@@ -562,8 +562,16 @@ int lee_get_info(lee_ctx* c, lee_info* info) {
   for (const auto& b : c->blk) info->increment_step &= increment_step_applies(c, b) ? 1 : 0;
   info->batched = c->batch.active ? 1 : 0;
   if (c->batch.active) {
-    batch_shape(c->batch.sshape, &info->batch_stage_tile[0], &info->batch_stage_tile[1]);
-    batch_shape(c->batch.fshape, &info->batch_filter_tile[0], &info->batch_filter_tile[1]);
+    if (c->batch.plane && c->batch.pshape < 0) {
+      info->batch_stage_tile[0] = info->batch_filter_tile[0] = kPlaneCols;
+      info->batch_stage_tile[1] = kPlaneBatchTall;
+      info->batch_filter_tile[1] = kPlaneWarps * kPlaneBatchRows;
+    } else {
+      const int ss = c->batch.pshape >= 0 ? c->batch.pshape : c->batch.sshape;
+      const int fs = c->batch.pshape >= 0 ? c->batch.pshape : c->batch.fshape;
+      batch_shape(ss, &info->batch_stage_tile[0], &info->batch_stage_tile[1]);
+      batch_shape(fs, &info->batch_filter_tile[0], &info->batch_filter_tile[1]);
+    }
   }
   return LEE_OK;
 }

@@ -175,21 +175,14 @@ int plane_batch_filter(lee_ctx* c) {
   return LEE_OK;
 }
 
-// Setup of the batched path at lee_prepare: operand arrays, sponge fields, and the tile shapes
-// of the stage and filter launches picked by timing every candidate (right-hand-side-only
-// stage launches and filter launches into scratch buffers, so the state is left alone).
+// The strips' tile shapes of the stage and filter launches, picked by timing every candidate
+// (right-hand-side-only stage launches and filter launches into scratch buffers, so the state is
+// left alone).
 template <typename T>
-int batch_setup(lee_ctx* c) {
+int batch_tune_strips(lee_ctx* c) {
   auto& bt = c->batch;
   const int nbk = (int)c->blk.size();
-  const Tableau tb = tableau(c->cfg.rk_scheme);
   int rc;
-  for (auto& b : c->blk)
-    if (!b.d_sigma_field && (rc = build_sigma_field(c, b))) return rc;
-  const size_t pbytes = sizeof(StageParams<T>) * (size_t)tb.ns * nbk;
-  if ((rc = dev_alloc(c, &bt.d_prm_graph, pbytes)) || (rc = dev_alloc(c, &bt.d_prm_direct, pbytes))) return rc;
-  std::vector<BatchFilterInst<T>> fi = batch_filter_inst<T>(c, false);
-  if ((rc = dev_alloc(c, &bt.d_finst, fi.size() * sizeof(fi[0])))) return rc;
   // scratch operands for the timing runs
   const std::vector<double> dts((size_t)nbk, 1e-3);
   std::vector<StageParams<T>> pr = batch_params<T>(c, dts, false, 1);
@@ -252,8 +245,23 @@ int batch_setup(lee_ctx* c) {
   CK(cudaMemcpyAsync(bt.d_ftiles, tiles_f.data(), tiles_f.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
   bt.nst = (int)tiles_s.size();
   bt.nft = (int)tiles_f.size();
+  return LEE_OK;
+}
+
+// Setup of the batched path at lee_prepare: operand arrays, sponge fields, work lists.
+template <typename T>
+int batch_setup(lee_ctx* c) {
+  auto& bt = c->batch;
+  const int nbk = (int)c->blk.size();
+  const Tableau tb = tableau(c->cfg.rk_scheme);
+  int rc;
+  for (auto& b : c->blk)
+    if (!b.d_sigma_field && (rc = build_sigma_field(c, b))) return rc;
+  const size_t pbytes = sizeof(StageParams<T>) * (size_t)tb.ns * nbk;
+  if ((rc = dev_alloc(c, &bt.d_prm_graph, pbytes)) || (rc = dev_alloc(c, &bt.d_prm_direct, pbytes))) return rc;
+  if ((rc = dev_alloc(c, &bt.d_finst, sizeof(BatchFilterInst<T>) * (size_t)nbk))) return rc;
   // the direct kernels serve every batch whose rows are 16-byte multiples (the row pitch's doing);
-  // the strips above run when lee_set_batch_shapes or lee_set_batch_persistent asks for them
+  // the strips run when lee_set_batch_shapes or lee_set_batch_persistent asks for them
   bt.plane = true;
   bt.jm_fields = false;
   for (auto& b : c->blk) {
@@ -268,8 +276,9 @@ int batch_setup(lee_ctx* c) {
     if ((rc = dalloc(c, &bt.d_maps, c->blk.size() * 4))) return rc;
     bt.npst = (int)ps.size();
     bt.npft = (int)pf.size();
+  } else if ((rc = batch_tune_strips<T>(c))) {
+    return rc;
   }
-  // the timing runs wrote right-hand sides and filtered values into scratch buffers only
   bt.active = true;
   return batch_refresh<T>(c);
 }

@@ -287,8 +287,8 @@ typedef struct {
   int stage_chunk;           /* planes marched per CTA by the stage kernel (autotuned; block 0) */
   int filter_chunk;          /* planes marched per CTA by the filter kernel (autotuned; block 0) */
   int batched;               /* 1 when the blocks run through the batched kernels */
-  int batch_stage_tile[2];   /* tile (xi, eta points) of the batched stage and filter launches, */
-  int batch_filter_tile[2];  /* picked by timing the candidates at lee_prepare */
+  int batch_stage_tile[2];   /* tile (xi, eta points) that the batched stage and filter launches */
+  int batch_filter_tile[2];  /* run: the default kernels', or the strips' that replaced them */
   int filter_kernel;         /* fused filter of block 0: 0 scalar, else the vector group width */
   int stage_kernel;          /* TMA stage kernel of block 0: points per thread */
   int filter_rows;           /* scalar fused filter of block 0: its form (lee_set_filter_form) */

@@ -97,3 +97,16 @@ def test_maps_of_later_buffers_and_contexts(product_lib, precision):
         tol = 1e-12 if precision == api.FP64 else 1e-6
         assert all(api.rel_l2(g, t.download(q)[0]) <= tol for q, g in enumerate(got))
         t.close()
+
+
+def test_info_reports_the_tiles_that_run(product_lib):
+    s = api.Solver(product_lib, _batch())
+    tiles = lambda: (tuple(s.info().batch_stage_tile), tuple(s.info().batch_filter_tile))
+    assert tiles() == ((64, 8), (64, 16))
+    assert product_lib.set_batch_persistent(s.ctx, 1) == api.LEE_OK
+    strip = tiles()
+    assert strip[0] == strip[1] and strip != ((64, 8), (64, 16))
+    assert product_lib.set_batch_persistent(s.ctx, -1) == api.LEE_OK
+    assert tiles() == ((64, 8), (64, 16))
+    assert product_lib.set_batch_shapes(s.ctx, 1, 0) == api.LEE_OK
+    assert tiles()[0] == strip[0] and tiles()[1] != strip[1]
