@@ -698,8 +698,10 @@ template <typename T, bool COMP, int TR>
 cudaError_t go_stage(const PlaneStage<T>& p, cudaStream_t s) {
   const dim3 grid((p.s.nx + kPlaneCols - 1) / kPlaneCols, (p.s.ny + kPlaneRows - 1) / kPlaneRows);
   const dim3 blk(32, kPlaneRows);
-  return launch<PlaneStage<T>>(p.s.code[0] ? k_plane_stage<T, COMP, TR, true> : k_plane_stage<T, COMP, TR, false>, grid,
-                               blk, p, s);
+  if (p.s.code[0]) return launch<PlaneStage<T>>(k_plane_stage<T, COMP, TR, true>, grid, blk, p, s);
+  // (a varying mean flow without holes runs the TMA kernels)
+  if constexpr ((TR & kTrUniform) != 0) return launch<PlaneStage<T>>(k_plane_stage<T, COMP, TR, false>, grid, blk, p, s);
+  return cudaErrorInvalidValue;
 }
 
 constexpr int kBase = kTrTma | kTrSponge;
