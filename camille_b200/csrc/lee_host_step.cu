@@ -423,7 +423,10 @@ int advance_impl(lee_ctx* c, int nsteps, const std::vector<double>& dts) {
   if (!g.one.exec) return direct(nsteps - done);
   // a replay ends before the next begins: 1.5 us between the steps of 20 us of a small block. Long
   // calls replay several periods at once, of up to 64 launches (256 x 256 FP64, five launches a
-  // step: 18.9 us a step by one, 17.2 by four, 16.2 by ten, 16.2 by twenty)
+  // step: 18.9 us a step by one, 17.2 by four, 16.2 by ten, 16.2 by twenty). The second capture costs
+  // the first call of a time step 0.4 ms, which its own steps give back from about 150 of them (first
+  // call and the next, us: 127 steps 2530 and 2378, 128 steps 2618 and 2129, 160 steps 3060 and 2629
+  // where 127's rate gives 3187 and 2996; 64 x 48 FP64 and 513 x 385 FP32 within 4 % of that)
   constexpr int kManySteps = 128;
   const int periods = (int)std::min<long long>(10, 64 / std::max<long long>(1, g.one.launches));
   if (!g.many.exec && periods > 1 && nsteps - done >= kManySteps) {

@@ -347,10 +347,13 @@ int lee_set_wait_limit(lee_ctx *ctx, double seconds);
 /* Kernel of the fused filter (no reference counterpart; results agree to rounding): -1 or 0
  * (default) the scalar kernel, 2 or 4 the kernel that gives each thread that many neighbouring
  * points along xi (4: FP32 only). LEE_ERR_UNSUPPORTED from lee_prepare when a block cannot run the
- * choice. Call before lee_prepare. */
+ * choice. Call before lee_prepare.
+ * This choice and the two below are refused on blocks whose rows are whole multiples of 16 bytes. On
+ * other blocks (an odd nxi, say) a choice that the block cannot run leaves it with its default, as
+ * these choices always did there; lee_info reports what block 0 runs. */
 int lee_set_filter_kernel(lee_ctx *ctx, int kind);
 /* Form of the scalar fused filter (no reference counterpart; all forms give the same bits):
- * 0 (default) the fastest form, timed at lee_prepare; 1 one tile row per thread on tiles of 8
+ * 0 (default) the fastest form, timed at lee_prepare (most 2-D blocks: a direct kernel); 1 one tile row per thread on tiles of 8
  * rows; 2 two rows per thread on tiles of 16 rows; 3 two neighbouring points of two rows per
  * thread on tiles of 64 x 16 points (packed FP32 arithmetic: the compensated form on 3-D blocks).
  * Forms 2 and 3 take no block with holes and not the vector kernel, form 3 nothing else
@@ -360,8 +363,10 @@ int lee_set_filter_form(lee_ctx *ctx, int form);
 /* Kernel of the RK stages on blocks that run the TMA stage kernel (no reference counterpart;
  * results agree to rounding): 1 one point per thread, 2 two neighbouring points per thread with
  * packed FP32 arithmetic (compensated form, uniform mean flow); -1 (default) takes 2
- * where it applies, and on blocks with a varying mean flow and no holes, else 1. LEE_ERR_UNSUPPORTED from lee_prepare when a block cannot run the
- * choice. Call before lee_prepare. */
+ * where it applies, and on blocks with a varying mean flow and no holes, else 1; most 2-D blocks with
+ * a uniform mean flow or holes run a direct kernel with the same bits instead. LEE_ERR_UNSUPPORTED
+ * from lee_prepare when a block cannot run the choice (see lee_set_filter_kernel). Call before
+ * lee_prepare. */
 int lee_set_stage_kernel(lee_ctx *ctx, int kind);
 
 /* ---- discrete adjoint (no reference counterpart: the reference has no adjoint) ----------
