@@ -382,8 +382,9 @@ int autotune(lee_ctx* c, BlockData& b) {
     // x 128); below about 40^3 its 64 x 16 tiles are too few (20^3 FP32 14.8 us against 12.7)
     const int nry = which == 1 && b.filter_form == 0 ? 3 : 1;
     // the ladder for every form, then the filter's other splits for the form that won there (a
-    // third of the launches of every split for every form: 12 instead of 40 ms at 129 x 113 x 97);
-    // on a small block, where the best chunks are shorter than the ladder's, every split for every form
+    // third of the launches of every split for every form: 12 instead of 40 ms at 129 x 113 x 97),
+    // where form 3 applies the others at two chunks (5 ms less); on a small block, where the best
+    // chunks are shorter than the ladder's, every split for every form
     int best_kq = 0;
     for (int phase = 0; phase < (d3 && which == 1 ? 2 : 1); ++phase) {
       for (int kq = 0; kq < (which == 1 ? nkinds : nskinds) * nry; ++kq) {
@@ -404,6 +405,8 @@ int autotune(lee_ctx* c, BlockData& b) {
         }
         for (int ch : (d3 ? (phase == 1 ? splits : ladder) : cands2)) {
           if (d3 && ch > b.nz) continue;
+          if (which == 1 && phase == 0 && !small && nry == 3 && b.filter_pair_ok && !b.filter_pair && ch != 32 && ch != 64)
+            continue;
           float ms = 0.f;
           for (int rep = 0; rep <= launches; ++rep) {  // the first run warms up
             if (rep == 1) CK(cudaEventRecord(e0, c->stream));
