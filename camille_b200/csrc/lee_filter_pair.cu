@@ -26,12 +26,16 @@
 // Each thread keeps its pair's xi weights (one closure class per point) in registers; rows near an
 // eta end (one warp each) and planes near a zeta end take their class rows.
 //
-// Bound by instruction issue (one row per thread: 292 instructions per pair and plane, 78 % of the
-// issue slots; the bytes take 208 us at 256^3). Two rows share the wait, the barrier, the addresses,
-// the classes and the eta window, and a tile of 16 rows filters half a halo row per own row instead
-// of one: 429 -> 355 us at 256^3, 49 -> 37 at 128 x 112 x 96; the zeta queue shifted every third
-// plane (its entries are addressed statically in between): 350 and 36. FP64 (one point of each row,
-// no increments) against k_filter_tma with two rows per thread, whose weights along eta and queues of
+// Bound by the latencies that 16 warps per SM leave open (192^3 FP32: 60 % of the issue slots, the
+// shared-memory pipe 53 %, DRAM 40 %; the bytes take 208 us at 256^3): one row per thread took 78 %
+// of the issue slots for 292 instructions per pair and plane. Two rows share the wait, the barrier,
+// the addresses, the classes and the eta window, and a tile of 16 rows filters half a halo row per
+// own row instead of one: 90 instructions per point and field instead of 152, 429 -> 355 us at
+// 256^3, 49 -> 37 at 128 x 112 x 96; the zeta queue shifted every third plane (its entries are
+// addressed statically in between): 350 and 36. Small and very narrow blocks have too few of the
+// 64 x 16 tiles (20^3 FP32 14.8 us, one row and one point 12.7; 16 x 400 x 300 takes that form too):
+// lee_prepare times the forms. FP64 (one point of each row, no increments; 47 % of the issue slots,
+// shared memory 64 %) against k_filter_tma with two rows per thread, whose weights along eta and queues of
 // pre-filter values and increments shift every plane: 189 -> 129 us at 160 x 144 x 128.
 //
 // Every mbarrier wait is bounded (about one second, or the context's limit); on expiry the CTA

@@ -14,9 +14,10 @@
 // With a non-uniform mean flow 21 coefficient pairs more are read per pair of points, without
 // branches (StageParams::mean), when the plane begins, so that they are in flight during the wait
 // and the derivatives. Held together with the inputs of the next plane they take up to 250
-// registers: two CTAs of 128 threads per SM. Bound by memory (220 bytes per point with all
-// coefficients fields: 47 us at 128 x 112 x 96); there 53 us per launch, the one-point kernel 134
-// with a branch per coefficient and 141 without (80 registers, spills).
+// registers: two CTAs of 128 threads per SM, whose eight warps leave latencies open (192 x 160 x 128:
+// a third of the issue slots, DRAM 51 %). A sheared mean flow on a curvilinear grid at 128 x 112 x 96
+// (17 coefficient fields and the sponge's, 167 bytes per point: 36 us): 53 us per launch, the
+// one-point kernel 134 with a branch per coefficient and 141 without (80 registers, spills).
 //
 // Every mbarrier wait is bounded (about one second); on expiry the CTA records the failure in the
 // device flag, waits (bounded) for its own copies in flight and returns.

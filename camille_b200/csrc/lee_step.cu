@@ -79,7 +79,8 @@ __global__ void __launch_bounds__(256) k_stage(StageParams<T> p) {
 // compile time, and a point's window along a line is its 11 points moved into the line, with the
 // weights of its closure class (0 interior, 1..5 left, 6..10 right rows) from shared memory, so
 // that boundary and interior points of a warp run the same instructions. Bound by the 165 cached
-// loads per point (FP64: 32 us of L1 bandwidth at 96^3); 128 threads, five CTAs per SM for the
+// loads per point (FP64: 32 us of L1 bandwidth at 96^3; 128^3: the L1 data pipe 74 %, warps waiting
+// on it); 128 threads, five CTAs per SM for the
 // uniform mean flow: 75 us per launch at 96^3 FP64, with four CTAs 80, six 78, and 88 with 256
 // threads (any shape of tile in j and k is within 3 %); k_stage, whose loops over the operator run
 // to a length read at run time, 213.
