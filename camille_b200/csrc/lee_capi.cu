@@ -612,8 +612,13 @@ int lee_get_setup(lee_ctx* c, int b, int what, double* out) {
   } else if (what == LEE_SETUP_JACOBIAN) {
     CK(cudaMemcpyAsync(out, bk.d_jac, N * 8, cudaMemcpyDeviceToHost, c->stream));
   } else if (what == LEE_SETUP_MEAN_GRADIENT) {
-    for (int q = 0; q < 5 * c->cfg.num_dim; ++q)
-      CK(cudaMemcpyAsync(out + q * N, bk.d_grad[q], N * 8, cudaMemcpyDeviceToHost, c->stream));
+    for (int q = 0; q < 5 * c->cfg.num_dim; ++q) {
+      if (bk.d_grad[q])
+        CK(cudaMemcpyAsync(out + q * N, bk.d_grad[q], N * 8, cudaMemcpyDeviceToHost, c->stream));
+      else
+        CK(cudaMemcpy2DAsync(out + q * N, (size_t)bk.nx * 8, gradient_copy(bk, c->cfg.num_dim, q), (size_t)bk.px * 8,
+                             (size_t)bk.nx * 8, (size_t)bk.ny * bk.nz, cudaMemcpyDeviceToHost, c->stream));
+    }
   } else if (what == LEE_SETUP_SPONGE) {
     CK(cudaStreamSynchronize(c->stream));
     memset(out, 0, N * 8);

@@ -334,6 +334,7 @@ bool is_bc_line(int kind);
 bool reads_inward(int kind);
 bool reads_wave(int kind);
 int dev_alloc(lee_ctx* c, void** p, size_t bytes);
+int dev_free(lee_ctx* c, void* p, size_t bytes);
 bool make_fd(OpTable* o, int scheme, int order);
 bool make_filter(OpTable* o, int scheme, int order, double strength);
 OpTable minus_identity(const OpTable& f);
@@ -367,6 +368,7 @@ template <typename T>
 int build_mean(lee_ctx* c, BlockData& b);
 template <typename T>
 void mean_coefs(const BlockData& b, Coef<T> (&k)[20]);
+const double* gradient_copy(const BlockData& b, int dim, int q);
 void set_pitch(const lee_ctx* c, BlockData& b);
 template <typename T>
 int run_filter(lee_ctx* c, BlockData& b, void** in, void** err, void** comp_out, void** f0, void** f1,

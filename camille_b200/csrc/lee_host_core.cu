@@ -94,6 +94,16 @@ int dev_alloc(lee_ctx* c, void** p, size_t bytes) {
   return LEE_OK;
 }
 
+// Give back an allocation of dev_alloc before the context ends.
+int dev_free(lee_ctx* c, void* p, size_t bytes) {
+  const auto it = std::find(c->allocs.begin(), c->allocs.end(), p);
+  if (it == c->allocs.end()) return LEE_OK;
+  CK(cudaFree(p));
+  c->allocs.erase(it);
+  c->device_bytes -= (long long)bytes;
+  return LEE_OK;
+}
+
 // Coefficient tables (src/solver/spatial_discretization.cpp:28-492); the numbers are the
 // published tables (Lele 1992; Bogey & Bailly 2004; Berland et al. 2007).
 bool make_fd(OpTable* o, int scheme, int order) {

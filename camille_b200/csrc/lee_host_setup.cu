@@ -52,6 +52,13 @@ int at_pitch(lee_ctx* c, const BlockData& b, P* in, P fill, P** out) {
 
 namespace lee {
 
+// The FP64 copy, at the row pitch, of the q-th mean gradient (field q / dim along q % dim), if its
+// coefficient is a field.
+const double* gradient_copy(const BlockData& b, int dim, int q) {
+  const int v = q / dim, x = q % dim;
+  return (v == 0 ? b.cd_gs[x] : v == 4 ? b.cd_gp[x] : b.cd_gu[(v - 1) * 3 + x]).p;
+}
+
 // The row pitch of a block's time-loop arrays: nx, or where nx values are no whole number of 16
 // bytes and the TMA-staged stage or filter kernel would run but for that (a tensor map's rows
 // start on 16 bytes), nx rounded up to one. At 129 x 113 x 97 in FP32 the step went from 1.11 to
@@ -231,7 +238,6 @@ int lee_prepare(lee_ctx* c) {
       CK(cudaStreamSynchronize(s));
       if ((rc = at_pitch(c, b, b.d_iblank, 0, &b.d_tiblank))) return rc;
     }
-    if ((rc = at_pitch(c, b, b.d_mean[4], 1.0, &b.d_tpbar))) return rc;
     // hole closures (receivers alone leave every closure as it is)
     if (b.has_holes) {
       std::vector<int8_t> code;
@@ -268,6 +274,8 @@ int lee_prepare(lee_ctx* c) {
         }
         CK(setup_scale(N, b.d_grad[v * dim + j], sum, b.d_jac, s));
       }
+    CK(cudaStreamSynchronize(s));
+    if ((rc = dev_free(c, sum, (size_t)N * 8)) || (rc = dev_free(c, tmp, (size_t)N * 8))) return rc;
     // J * metrics products read by the stage kernels
     for (int l = 0; l < dim; ++l)
       for (int x = 0; x < dim; ++x) {
@@ -437,10 +445,31 @@ int lee_prepare(lee_ctx* c) {
     }
     b.need_rho = 0;
     for (int q = 0; q < 9; ++q) b.need_rho |= c->comp ? !b.cf_gu[q].zero : !b.cd_gu[q].zero;
-    if (b.need_rho && (rc = dev_alloc(c, &b.rho, (size_t)b.NP * c->esz))) return rc;
+    if (b.need_rho) {
+      if ((rc = dev_alloc(c, &b.rho, (size_t)b.NP * c->esz))) return rc;
+      if ((rc = at_pitch(c, b, b.d_mean[4], 1.0, &b.d_tpbar))) return rc;
+    }
     b.rho_valid = false;
     if ((rc = c->comp ? build_mean<float>(c, b) : build_mean<double>(c, b))) return rc;
     if ((rc = scalar_setup(c, b))) return rc;
+    // padded rows: the coefficients are copies, and what nothing else reads of their sources goes back
+    // before the state is allocated, so that a block takes about the memory that an unpadded one does
+    // (lee_get_setup reads the mean gradients from the copies then)
+    if (b.px != b.nx) {
+      CK(cudaStreamSynchronize(s));
+      const size_t bytes = (size_t)N * 8;
+      for (int q = 0; q < 9; ++q) {
+        if ((rc = dev_free(c, b.d_jm[q], bytes))) return rc;
+        b.d_jm[q] = nullptr;
+      }
+      if ((rc = dev_free(c, b.d_rbi, bytes))) return rc;
+      b.d_rbi = nullptr;
+      for (int q = 0; q < 5 * dim && !c->comp; ++q) {
+        if (!gradient_copy(b, dim, q)) continue;
+        if ((rc = dev_free(c, b.d_grad[q], bytes))) return rc;
+        b.d_grad[q] = nullptr;
+      }
+    }
     // state buffers
     if ((rc = alloc_fields(c, b.y, b.NP))) return rc;
     if ((rc = alloc_fields(c, b.acc, b.NP))) return rc;
